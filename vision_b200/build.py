@@ -4,12 +4,13 @@ usage: python vision_b200/build.py [--force] [-v]
 
 Objects go to vision_b200/_build/; the shared library lands next to this file
 so that it travels with the package.  Each object and the library carry a
-digest of their sources, headers and flags (`.stamp` files); only objects
+digest of their sources, included headers and flags (`.stamp` files); only objects
 whose digest changed are recompiled, in parallel.
 """
 import concurrent.futures
 import hashlib
 import os
+import re
 import subprocess
 import sys
 
@@ -21,7 +22,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), 'include')
 
 SOURCES = ['kernels.cu', 'wavefront.cu', 'restir.cu', 'restir_diffuse.cu', 'svgf.cu', 'server.cu', 'mlp.cu', 'cache_render.cu', 'capi.cu', 'noalloc.cu', 'scene_load.cpp', 'image_io.cpp', 'bvh8.cpp', 'rgb2spec.cpp', 'luts.cpp', 'lut_gen.cu']
 ARCH = ['-gencode', 'arch=compute_100a,code=sm_100a']
-COMMON = ['-O3', '-std=c++17', '-lineinfo', '-Xcompiler', '-fPIC,-ffp-contract=off,-pthread',
+COMMON = ['-O3', '-std=c++17', '-lineinfo', '-Xptxas', '--split-compile=0', '-Xcompiler', '-fPIC,-ffp-contract=off,-pthread',
           '-I', CSRC, '-I', INCLUDE]
 # Per-source device flags.  svgf.cu: no multiply-add contraction, as in the
 # host oracle; its edge-stopping weights (exp of depth and luminance
@@ -55,8 +56,22 @@ def _headers():
     return sorted(hs)
 
 
+def _includes(path, seen):
+    """The quoted includes of a file, transitively (those found in csrc/ or include/)."""
+    with open(path) as f:
+        names = re.findall(r'^\s*#\s*include\s+"([^"]+)"', f.read(), re.M)
+    for n in names:
+        for d in (CSRC, INCLUDE):
+            p = os.path.join(d, n)
+            if os.path.exists(p) and p not in seen:
+                seen.add(p)
+                _includes(p, seen)
+    return seen
+
+
 def _source_digest(src):
-    return _digest([os.path.join(CSRC, src)] + _headers(), ARCH + COMMON + SOURCE_FLAGS.get(src, []))
+    path = os.path.join(CSRC, src)
+    return _digest([path] + sorted(_includes(path, set())), ARCH + COMMON + SOURCE_FLAGS.get(src, []))
 
 
 def _library_digest():
