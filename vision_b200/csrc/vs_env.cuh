@@ -43,7 +43,7 @@ __device__ __forceinline__ Spec<N> env_L(const DeviceScene &s, float u, float v,
     rgb2spec_unbound(s.rgb2spec, rgb, c);
 #pragma unroll
     for (int i = 0; i < N; ++i)
-        r.v[i] = sigmoid_poly(c[0], c[1], c[2], wl.lambda[i]) * c[3] * cie_spd(c_spec.d65, wl.lambda[i]) * s.env.scale;
+        r.v[i] = sigmoid_poly(c[0], c[1], c[2], wl.lambda[i]) * c[3] * cie_d65(wl.lambda[i]) * s.env.scale;
     return r;
 }
 

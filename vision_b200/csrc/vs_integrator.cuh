@@ -151,7 +151,7 @@ __device__ __forceinline__ Spec<N> projector_L(const DeviceScene &s, const AreaL
     rgb2spec_unbound(s.rgb2spec, rgb, c);
 #pragma unroll
     for (int i = 0; i < N; ++i)
-        r.v[i] = sigmoid_poly(c[0], c[1], c[2], wl.lambda[i]) * c[3] * cie_spd(c_spec.d65, wl.lambda[i]) * L.scale / d2;
+        r.v[i] = sigmoid_poly(c[0], c[1], c[2], wl.lambda[i]) * c[3] * cie_d65(wl.lambda[i]) * L.scale / d2;
     return r;
 }
 
