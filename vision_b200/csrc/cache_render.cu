@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(128) k_cache_paths(const __grid_constant__ Dev
         else ret += linear_srgb<CN>(c, wl);
     };
     for (uint32_t bounce = 0; bounce <= end_depth; ++bounce) {
-        RayPre rp = precompute_ray(ro, rd);
+        RayPre rp = precompute_ray(ro, rd, s.bound);
         Hit hit;
         float t_hit;
         const bool hit_any = trace_closest(s, rp, 3.402823466e+38f, hit, t_hit);
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(128) k_cache_paths(const __grid_constant__ Dev
         f2 u_surf = smp.next2();
         LightSample<CN> ls = sample_light<CN>(s, it, u_light, u_surf, wl);
         Ray sh = spawn_ray_to(it.pos, it.ng, ls.p_light);
-        bool occluded = trace_any(s, precompute_ray(sh.o, sh.d), sh.tmax);
+        bool occluded = trace_any(s, precompute_ray(sh.o, sh.d, s.bound), sh.tmax);
         Material mat = s.materials[it.mat];
         Bsdf<CN> bsdf = make_bsdf<CN>(s, mat, it.shading, it.ng, it.wo, it.uv, wl);
         if (bsdf.dispersive) invalidate_secondary<CN>(wl);
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(128) k_cw_generate(const __grid_constant__ Dev
 }
 
 template <int L>
-__global__ void __launch_bounds__(128) k_cw_extend(const __grid_constant__ DeviceScene s,
+__global__ void __launch_bounds__(128, traverse_blocks(L)) k_cw_extend(const __grid_constant__ DeviceScene s,
                                                    const __grid_constant__ WfBuffers b, uint32_t cur) {
     wf::extend<L>(CacheScene{&s}, b, cur);
 }
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(128) k_cw_shade(const __grid_constant__ Device
 }
 
 template <int L>
-__global__ void __launch_bounds__(128) k_cw_shadow(const __grid_constant__ DeviceScene s,
+__global__ void __launch_bounds__(128, traverse_blocks(L)) k_cw_shadow(const __grid_constant__ DeviceScene s,
                                                    const __grid_constant__ WfBuffers b, float4 *ended) {
     wf::shadow<L>(CacheScene{&s}, b, 0, ended);
 }
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(128) k_cache_suffix(const __grid_constant__ De
             ++ps.bounce;
             Hit h;
             float t_hit;
-            const bool hit_any = trace_closest(s, precompute_ray(ps.ro, ps.rd), 3.402823466e+38f, h, t_hit);
+            const bool hit_any = trace_closest(s, precompute_ray(ps.ro, ps.rd, s.bound), 3.402823466e+38f, h, t_hit);
             if (ps.bounce == end_depth) {
                 if (!hit_any) {
                     miss_emission<CN>(s, ps, acc);

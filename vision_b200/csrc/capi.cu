@@ -354,6 +354,11 @@ struct vs_scene {
         d.filter_integral = host.filter_integral;
         d.cam = host.cam;
         d.ip = host.ip;
+        if (!host.nodes.empty()) {
+            const Bvh8Node &n = host.nodes[0];
+            d.bound = {std::fabs(n.px) + std::ldexp(256.0f, n.e[0] - 127), std::fabs(n.py) + std::ldexp(256.0f, n.e[1] - 127),
+                       std::fabs(n.pz) + std::ldexp(256.0f, n.e[2] - 127)};
+        }
         d.node_count = static_cast<uint32_t>(host.nodes.size());
         d.prim_count = static_cast<uint32_t>(host.prim_inst.size());
         d.two_level = host.two_level ? 1u : 0u;

@@ -24,7 +24,7 @@ __global__ void __launch_bounds__(128) k_trace_closest(const __grid_constant__ D
     if (i >= n) return;
     const float4 *r4 = reinterpret_cast<const float4 *>(rays) + 2u * i;
     float4 a = r4[0], b = r4[1];
-    RayPre rp = precompute_ray(make3(a.x, a.y, a.z), make3(b.x, b.y, b.z));
+    RayPre rp = precompute_ray(make3(a.x, a.y, a.z), make3(b.x, b.y, b.z), s.bound);
     float tmax = b.w;
     Hit h;
     float t;
@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(128) k_trace_any(const __grid_constant__ Devic
     if (i >= n) return;
     const float4 *r4 = reinterpret_cast<const float4 *>(rays) + 2u * i;
     float4 a = r4[0], b = r4[1];
-    RayPre rp = precompute_ray(make3(a.x, a.y, a.z), make3(b.x, b.y, b.z));
+    RayPre rp = precompute_ray(make3(a.x, a.y, a.z), make3(b.x, b.y, b.z), s.bound);
     occ[i] = trace_any(s, rp, b.w) ? 1u : 0u;
 }
 

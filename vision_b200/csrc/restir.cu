@@ -393,7 +393,7 @@ __device__ __forceinline__ float di_p_hat_at(const DeviceScene &s, const Interac
 
 __device__ __forceinline__ bool occluded_to(const DeviceScene &s, const Interaction &it, f3 p) {
     Ray sh = spawn_ray_to(it.pos, it.ng, p);
-    return trace_any(s, precompute_ray(sh.o, sh.d), sh.tmax);
+    return trace_any(s, precompute_ray(sh.o, sh.d, s.bound), sh.tmax);
 }
 
 // ReSTIRDI::compute_hit (direct.cpp:353-400): primary hit and its chain of
@@ -418,7 +418,7 @@ __device__ VS_OUTLINE PrimaryHit compute_hit(const DeviceScene &s, const RtParam
     for (;;) {
         Hit h;
         float t;
-        r.hit = trace_closest(s, precompute_ray(ro, rd), 3.402823466e+38f, h, t);
+        r.hit = trace_closest(s, precompute_ray(ro, rd, s.bound), 3.402823466e+38f, h, t);
         if (!r.hit) {
             r.surf.hit.inst_id = kInvalid;
             r.surf.hit.prim_id = kInvalid;
@@ -641,7 +641,7 @@ __device__ VS_OUTLINE DiReservoir di_ris(const DeviceScene &s, const RtParams &p
         Ray ray = di_bsdf_ray(it, bsdf, smp, hb);
         Hit h;
         float t;
-        bool hit = trace_closest(s, precompute_ray(ray.o, ray.d), ray.tmax, h, t);
+        bool hit = trace_closest(s, precompute_ray(ray.o, ray.d, s.bound), ray.tmax, h, t);
         DiReservoir cand;
         float weight;
         di_bsdf_candidate(s, p, it, wl, hb, hit, h, ray.d, lum_tp, cand, weight);
@@ -957,7 +957,7 @@ __global__ void __launch_bounds__(128, VS_RT_LIGHTS_MIN_BLOCKS)
 
 // Stage 3: the BSDF candidates' closest hits (warps refill finished lanes,
 // as the wavefront traversal kernels do).
-__global__ void __launch_bounds__(128) k_di_bsdf_trace(const __grid_constant__ DeviceScene s,
+__global__ void __launch_bounds__(128, kTraverseBlocks) k_di_bsdf_trace(const __grid_constant__ DeviceScene s,
                                                        const __grid_constant__ RtParams p,
                                                        const __grid_constant__ RtBuffers b) {
     if (p.M_bsdf != 1u) return;
@@ -973,7 +973,7 @@ __global__ void __launch_bounds__(128) k_di_bsdf_trace(const __grid_constant__ D
             if (k < n) {
                 idx = b.di_list[k];
                 const float4 o = b.di_ray[2ull * idx], d = b.di_ray[2ull * idx + 1];
-                r = precompute_ray(make3(o.x, o.y, o.z), make3(d.x, d.y, d.z));
+                r = precompute_ray(make3(o.x, o.y, o.z), make3(d.x, d.y, d.z), s.bound);
                 trav_init(t, r, o.w);
                 active = true;
             }
@@ -1022,7 +1022,7 @@ __global__ void __launch_bounds__(128, VS_RT_MIN_BLOCKS)
 
 // Stage 5: visibility of the chosen samples (an occluded sample keeps its
 // history count but loses its weight), with ray replacement.
-__global__ void __launch_bounds__(128) k_di_visibility(const __grid_constant__ DeviceScene s,
+__global__ void __launch_bounds__(128, kTraverseBlocks) k_di_visibility(const __grid_constant__ DeviceScene s,
                                                        const __grid_constant__ RtBuffers b) {
     const uint32_t n = *b.di_count;
     uint2 stack[kStackSize];
@@ -1036,7 +1036,7 @@ __global__ void __launch_bounds__(128) k_di_visibility(const __grid_constant__ D
             if (k < n) {
                 idx = b.di_list[k];
                 const float4 o = b.di_ray[2ull * idx], d = b.di_ray[2ull * idx + 1];
-                r = precompute_ray(make3(o.x, o.y, o.z), make3(d.x, d.y, d.z));
+                r = precompute_ray(make3(o.x, o.y, o.z), make3(d.x, d.y, d.z), s.bound);
                 trav_init(t, r, o.w);
                 active = true;
             }
@@ -1195,7 +1195,7 @@ __global__ void __launch_bounds__(128, VS_RT_MIN_BLOCKS)
 
 // Shading rays of the listed pixels (ray replacement); w of the direction
 // record becomes 1 when the ray is occluded.
-__global__ void __launch_bounds__(128) k_di_sp_vis(const __grid_constant__ DeviceScene s,
+__global__ void __launch_bounds__(128, kTraverseBlocks) k_di_sp_vis(const __grid_constant__ DeviceScene s,
                                                    const __grid_constant__ RtBuffers b) {
     const uint32_t n = *b.di_count;
     uint2 stack[kStackSize];
@@ -1209,7 +1209,7 @@ __global__ void __launch_bounds__(128) k_di_sp_vis(const __grid_constant__ Devic
             if (k < n) {
                 idx = b.di_list[k];
                 const float4 o = b.di_ray[2ull * idx], d = b.di_ray[2ull * idx + 1];
-                r = precompute_ray(make3(o.x, o.y, o.z), make3(d.x, d.y, d.z));
+                r = precompute_ray(make3(o.x, o.y, o.z), make3(d.x, d.y, d.z), s.bound);
                 trav_init(t, r, o.w);
                 active = true;
             }
@@ -1452,12 +1452,12 @@ __global__ void __launch_bounds__(128) k_gi_wf_shade(const __grid_constant__ Dev
     wf::shade<RN, C>(RtScene{&s}, w, cur, 0, radiance);
 }
 
-__global__ void __launch_bounds__(128) k_gi_wf_extend(const __grid_constant__ DeviceScene s,
+__global__ void __launch_bounds__(128, kTraverseBlocks) k_gi_wf_extend(const __grid_constant__ DeviceScene s,
                                                       const __grid_constant__ WfBuffers w, uint32_t cur) {
     wf::extend<kLevelsFlat>(RtScene{&s}, w, cur);
 }
 
-__global__ void __launch_bounds__(128) k_gi_wf_shadow(const __grid_constant__ DeviceScene s,
+__global__ void __launch_bounds__(128, kTraverseBlocks) k_gi_wf_shadow(const __grid_constant__ DeviceScene s,
                                                       const __grid_constant__ WfBuffers w, float4 *radiance) {
     wf::shadow<kLevelsFlat>(RtScene{&s}, w, 0, radiance);
 }
@@ -1616,7 +1616,7 @@ __global__ void __launch_bounds__(128, VS_RT_MIN_BLOCKS)
 }
 
 // Visibility of the queued neighbour samples (ray replacement).
-__global__ void __launch_bounds__(128) k_gi_sp_vis(const __grid_constant__ DeviceScene s,
+__global__ void __launch_bounds__(128, kTraverseBlocks) k_gi_sp_vis(const __grid_constant__ DeviceScene s,
                                                    const __grid_constant__ RtBuffers b) {
     const uint32_t n = b.gs_count[0];
     uint2 stack[kStackSize];
@@ -1630,7 +1630,7 @@ __global__ void __launch_bounds__(128) k_gi_sp_vis(const __grid_constant__ Devic
             if (k < n) {
                 e = b.gs_list[k];
                 const float4 o = b.gs_ray[2ull * e], d = b.gs_ray[2ull * e + 1];
-                r = precompute_ray(make3(o.x, o.y, o.z), make3(d.x, d.y, d.z));
+                r = precompute_ray(make3(o.x, o.y, o.z), make3(d.x, d.y, d.z), s.bound);
                 trav_init(t, r, o.w);
                 active = true;
             }

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(256) k_svgf_geom(const __grid_constant__ Devic
     f2 mv = make2(0.0f, 0.0f);
     Hit h;
     float t;
-    if (trace_closest(s, precompute_ray(ro, rd), 3.402823466e+38f, h, t)) {
+    if (trace_closest(s, precompute_ray(ro, rd, s.bound), 3.402823466e+38f, h, t)) {
         const Interaction it = surface_interaction(s, h, rd, true);
         const f3 n = it.shading.z;
         g.nx = n.x;

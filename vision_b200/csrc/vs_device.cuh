@@ -321,60 +321,77 @@ VS_HD Ray spawn_ray_to(f3 pos, f3 ng, f3 target) {
 // GPU and in the CPU oracle.  Barycentrics: u weights vertex 1, v vertex 2.
 // ---------------------------------------------------------------------------
 struct RayPre {
+    // Triangle test: origin and shear in the ray's axis order (kz: dominant
+    // direction component, then kx = kz + 1, ky = kz + 2 modulo 3).
     f3 o;
-    f3 d;
-    f3 inv_d;
-    int kx, ky, kz;
     float sx, sy, sz;
-    uint32_t oct;  // bit i set when d[i] < 0
+    int kz;
+    // Box test, in world axes: reciprocal direction, and -o / d less (near
+    // planes) and plus (far planes) the bound below on its rounding errors.
+    f3 inv_d;
+    f3 cn, cf;
+    uint32_t oct;  // bit i set when inv_d[i] < 0
+    f3 wo, wd;     // the ray in world axes (for instance transforms)
 };
 
-__device__ __forceinline__ RayPre precompute_ray(f3 o, f3 d) {
+// `bound`: the largest coordinate magnitude, per axis, of the BVH's boxes.
+//
+// The box distances of intersect_children are q * (2^e / d) + ((p - o) / d),
+// the second term as p / d + (-o / d).  Its roundings, those of the quantised
+// planes and those of the triangle test are each at most a few 2^-24 of
+// (|o| + |plane|) / |d|; cn and cf move every near plane down and every far
+// plane up by 2^-21 of that, so a box is entered whenever the float triangle
+// test can accept one of its triangles.  (1 / d is an approximation, good to
+// 2 ulp, for the same reason; the shear factors are exactly rounded.)
+__device__ __forceinline__ RayPre precompute_ray(f3 o, f3 d, f3 bound) {
     RayPre r;
-    r.o = o;
-    r.d = d;
+    r.wo = o;
+    r.wd = d;
     const float tiny = 1e-30f;
-    r.inv_d = {1.0f / (fabsf(d.x) > tiny ? d.x : copysignf(tiny, d.x)),
-               1.0f / (fabsf(d.y) > tiny ? d.y : copysignf(tiny, d.y)),
-               1.0f / (fabsf(d.z) > tiny ? d.z : copysignf(tiny, d.z))};
+    r.inv_d = {__fdividef(1.0f, fabsf(d.x) > tiny ? d.x : copysignf(tiny, d.x)),
+               __fdividef(1.0f, fabsf(d.y) > tiny ? d.y : copysignf(tiny, d.y)),
+               __fdividef(1.0f, fabsf(d.z) > tiny ? d.z : copysignf(tiny, d.z))};
+    const float k = 1.0f / 2097152.0f;
+    const f3 b = {-o.x * r.inv_d.x, -o.y * r.inv_d.y, -o.z * r.inv_d.z};
+    const f3 e = {k * (bound.x + fabsf(o.x)) * fabsf(r.inv_d.x), k * (bound.y + fabsf(o.y)) * fabsf(r.inv_d.y),
+                  k * (bound.z + fabsf(o.z)) * fabsf(r.inv_d.z)};
+    r.cn = b - e;
+    r.cf = b + e;
     float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
-    int kz = (ax > ay) ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);
-    int kx = kz + 1 == 3 ? 0 : kz + 1;
-    int ky = kx + 1 == 3 ? 0 : kx + 1;
-    if (comp(d, kz) < 0.0f) {
-        int t = kx; kx = ky; ky = t;
-    }
-    r.kx = kx; r.ky = ky; r.kz = kz;
-    float dz = comp(d, kz);
+    r.kz = (ax > ay) ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);
+    const int kx = r.kz == 2 ? 0 : r.kz + 1;
+    const int ky = kx == 2 ? 0 : kx + 1;
+    r.o = {comp(o, kx), comp(o, ky), comp(o, r.kz)};
+    const float dz = comp(d, r.kz);
     r.sx = __fdiv_rn(comp(d, kx), dz);
     r.sy = __fdiv_rn(comp(d, ky), dz);
     r.sz = __fdiv_rn(1.0f, dz);
-    r.oct = (d.x < 0.0f ? 1u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 4u : 0u);
+    r.oct = (r.inv_d.x < 0.0f ? 1u : 0u) | (r.inv_d.y < 0.0f ? 2u : 0u) | (r.inv_d.z < 0.0f ? 4u : 0u);
     return r;
 }
 
-__device__ __forceinline__ float pick(const float4 &v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
+// A vertex relative to the ray's origin, in its axis order.
+__device__ __forceinline__ f3 ray_axes(const RayPre &r, const float4 &v) {
+    const bool k0 = r.kz == 0, k1 = r.kz == 1;
+    return {__fsub_rn(k0 ? v.y : (k1 ? v.z : v.x), r.o.x), __fsub_rn(k0 ? v.z : (k1 ? v.x : v.y), r.o.y),
+            __fsub_rn(k0 ? v.x : (k1 ? v.y : v.z), r.o.z)};
+}
 
 // Returns true and fills (t, u, v) when the ray hits the triangle with
-// tmin < t < tmax.
+// tmin < t < tmax.  The published test swaps kx and ky for a negative dominant
+// component to keep the winding; the swap negates U, V, W, their sum and T
+// exactly, so t, u and v and every comparison below are the same without it
+// (up to the sign of a zero u or v, which is set at the end).
 __device__ __forceinline__ bool intersect_triangle(const RayPre &r, const float4 &v0, const float4 &v1,
                                                    const float4 &v2, float tmin, float tmax,
                                                    float &t_out, float &u_out, float &v_out) {
-    float ax = __fsub_rn(pick(v0, r.kx), comp(r.o, r.kx));
-    float ay = __fsub_rn(pick(v0, r.ky), comp(r.o, r.ky));
-    float az = __fsub_rn(pick(v0, r.kz), comp(r.o, r.kz));
-    float bx = __fsub_rn(pick(v1, r.kx), comp(r.o, r.kx));
-    float by = __fsub_rn(pick(v1, r.ky), comp(r.o, r.ky));
-    float bz = __fsub_rn(pick(v1, r.kz), comp(r.o, r.kz));
-    float cx = __fsub_rn(pick(v2, r.kx), comp(r.o, r.kx));
-    float cy = __fsub_rn(pick(v2, r.ky), comp(r.o, r.ky));
-    float cz = __fsub_rn(pick(v2, r.kz), comp(r.o, r.kz));
-    float Ax = __fsub_rn(ax, __fmul_rn(r.sx, az));
-    float Ay = __fsub_rn(ay, __fmul_rn(r.sy, az));
-    float Bx = __fsub_rn(bx, __fmul_rn(r.sx, bz));
-    float By = __fsub_rn(by, __fmul_rn(r.sy, bz));
-    float Cx = __fsub_rn(cx, __fmul_rn(r.sx, cz));
-    float Cy = __fsub_rn(cy, __fmul_rn(r.sy, cz));
+    const f3 a = ray_axes(r, v0), b = ray_axes(r, v1), c = ray_axes(r, v2);
+    float Ax = __fsub_rn(a.x, __fmul_rn(r.sx, a.z));
+    float Ay = __fsub_rn(a.y, __fmul_rn(r.sy, a.z));
+    float Bx = __fsub_rn(b.x, __fmul_rn(r.sx, b.z));
+    float By = __fsub_rn(b.y, __fmul_rn(r.sy, b.z));
+    float Cx = __fsub_rn(c.x, __fmul_rn(r.sx, c.z));
+    float Cy = __fsub_rn(c.y, __fmul_rn(r.sy, c.z));
     float U = __fsub_rn(__fmul_rn(Cx, By), __fmul_rn(Cy, Bx));
     float V = __fsub_rn(__fmul_rn(Ax, Cy), __fmul_rn(Ay, Cx));
     float W = __fsub_rn(__fmul_rn(Bx, Ay), __fmul_rn(By, Ax));
@@ -392,15 +409,25 @@ __device__ __forceinline__ bool intersect_triangle(const RayPre &r, const float4
     if ((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f)) return false;
     float det = __fadd_rn(__fadd_rn(U, V), W);
     if (det == 0.0f) return false;
-    float Az = __fmul_rn(r.sz, az);
-    float Bz = __fmul_rn(r.sz, bz);
-    float Cz = __fmul_rn(r.sz, cz);
+    float Az = __fmul_rn(r.sz, a.z);
+    float Bz = __fmul_rn(r.sz, b.z);
+    float Cz = __fmul_rn(r.sz, c.z);
     float T = __fadd_rn(__fadd_rn(__fmul_rn(U, Az), __fmul_rn(V, Bz)), __fmul_rn(W, Cz));
     float t = __fdiv_rn(T, det);
     if (!(t > tmin && t < tmax)) return false;
     t_out = t;
     u_out = __fdiv_rn(V, det);
     v_out = __fdiv_rn(W, det);
+    if (r.sz < 0.0f) {
+        // A zero V or W came from the products above; swapped, its sign is
+        // that of their difference the other way round.
+        if (V == 0.0f)
+            u_out = __fdiv_rn(static_cast<float>(static_cast<double>(Ay) * static_cast<double>(Cx) -
+                                                 static_cast<double>(Ax) * static_cast<double>(Cy)), -det);
+        if (W == 0.0f)
+            v_out = __fdiv_rn(static_cast<float>(static_cast<double>(By) * static_cast<double>(Ax) -
+                                                 static_cast<double>(Bx) * static_cast<double>(Ay)), -det);
+    }
     return true;
 }
 
@@ -423,68 +450,94 @@ constexpr float kBoxSlack = 1.000001f;
 // compares boxes against best_t plus this bound, so a box entered within the
 // error of the best hit (another triangle at the same t, as on an edge shared
 // next to the origin) is still opened.
-__device__ __forceinline__ float tri_t_error(const RayPre &r, const float4 &a, const float4 &b, const float4 &c) {
-    const float m = fmaxf(fmaxf(fmaxf(fabsf(a.x - r.o.x), fabsf(a.y - r.o.y)), fmaxf(fabsf(a.z - r.o.z), fabsf(b.x - r.o.x))),
-                          fmaxf(fmaxf(fabsf(b.y - r.o.y), fabsf(b.z - r.o.z)),
-                                fmaxf(fmaxf(fabsf(c.x - r.o.x), fabsf(c.y - r.o.y)), fabsf(c.z - r.o.z))));
+__device__ __forceinline__ float tri_t_error(const RayPre &r, const float4 &v0, const float4 &v1, const float4 &v2) {
+    const f3 a = ray_axes(r, v0), b = ray_axes(r, v1), c = ray_axes(r, v2);
+    const float m = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(b.x))),
+                          fmaxf(fmaxf(fabsf(b.y), fabsf(b.z)), fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fabsf(c.z))));
     return m * fabsf(r.sz) * (1.0f / 65536.0f);
 }
 
-struct NodeHits {
-    uint32_t internal_hits;  // bits 24..31: internal children in traversal order
-    uint32_t tri_hits;       // bits 0..23: triangles of the leaf children that were hit
-};
-
-__device__ __forceinline__ float ubyte(uint32_t w, int i) {
-    return static_cast<float>((w >> (8 * i)) & 0xffu);
+// Byte i of w, q, as the float 1 + q 2^-15: one byte permute.
+__device__ __forceinline__ float ubyte_biased(uint32_t w, uint32_t i) {
+    return __uint_as_float(__byte_perm(w, 0x3f800000u, 0x7604u | (i << 4)));
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
 }
 
 // Tests the 8 children of one node; returns the new node and triangle groups.
+//
+// Traversal is bound by instruction issue (the nodes hit L1 and L2), so the
+// test is written for few instructions per child: the near and far plane of
+// each axis are picked once per node by the ray's octant (no minimum and
+// maximum per axis and child), a plane distance is one byte permute and one
+// multiply-add, U * (1 + q 2^-15) + (base - U) with U = 2^15 2^e / d, and the
+// slab test is two three-input and two two-input minima and maxima.  Rounding
+// base - U costs at most 2^-9 grid steps, which 2^-7 steps of slack on each
+// side cover, besides cn and cf.  Empty slots hold zero boxes and zero meta
+// bytes and contribute no bits, so they are not skipped.
+// Measured, 2.1 M camera rays against 2.3 M triangles: 0.57 -> 0.41 ms; bounce
+// rays 0.54 -> 0.37 ms, shadow rays 0.43 -> 0.31 ms; 10,000 emitters in a room,
+// bounce rays 1.29 -> 0.87 ms (per-child reconstruction of both planes in
+// floats, minima and maxima per axis before; ray replacement on both sides).
+// Slower: both planes of an axis in one packed fma.rn.f32x2 (more registers),
+// byte-to-float conversions in place of the permute, 96-byte nodes fetched
+// with 32-byte loads, testing triangles only once 8 lanes have one.
 __device__ __forceinline__ void intersect_children(const uint4 *nodes, uint32_t node_index, const RayPre &r,
                                                    float tmax, uint2 &node_group, uint2 &tri_group) {
     const uint4 *np = nodes + static_cast<size_t>(node_index) * 5u;
-    uint4 w0 = __ldg(np + 0);
-    uint4 w1 = __ldg(np + 1);
-    uint4 w2 = __ldg(np + 2);
-    uint4 w3 = __ldg(np + 3);
-    uint4 w4 = __ldg(np + 4);
-    float px = __uint_as_float(w0.x), py = __uint_as_float(w0.y), pz = __uint_as_float(w0.z);
-    float sx = __uint_as_float((w0.w & 0xffu) << 23);
-    float sy = __uint_as_float(((w0.w >> 8) & 0xffu) << 23);
-    float sz = __uint_as_float(((w0.w >> 16) & 0xffu) << 23);
-    uint32_t imask = w0.w >> 24;
-    uint32_t qlox[2] = {w2.x, w2.y}, qloy[2] = {w2.z, w2.w}, qloz[2] = {w3.x, w3.y};
-    uint32_t qhix[2] = {w3.z, w3.w}, qhiy[2] = {w4.x, w4.y}, qhiz[2] = {w4.z, w4.w};
-    uint32_t meta[2] = {w1.z, w1.w};
-    uint32_t ihits = 0, thits = 0;
+    const uint4 w0 = __ldg(np + 0);
+    const uint4 w1 = __ldg(np + 1);
+    const uint4 w2 = __ldg(np + 2);
+    const uint4 w3 = __ldg(np + 3);
+    const uint4 w4 = __ldg(np + 4);
+    const float Ux = __uint_as_float((w0.w & 0xffu) << 23) * (r.inv_d.x * 32768.0f);
+    const float Uy = __uint_as_float(((w0.w >> 8) & 0xffu) << 23) * (r.inv_d.y * 32768.0f);
+    const float Uz = __uint_as_float(((w0.w >> 16) & 0xffu) << 23) * (r.inv_d.z * 32768.0f);
+    const uint32_t imask = w0.w >> 24;
+    const float px = __uint_as_float(w0.x), py = __uint_as_float(w0.y), pz = __uint_as_float(w0.z);
+    const float g = 1.0f / 4194304.0f;
+    const float bnx = fmaf(fabsf(Ux), -g, fmaf(px, r.inv_d.x, r.cn.x) - Ux);
+    const float bny = fmaf(fabsf(Uy), -g, fmaf(py, r.inv_d.y, r.cn.y) - Uy);
+    const float bnz = fmaf(fabsf(Uz), -g, fmaf(pz, r.inv_d.z, r.cn.z) - Uz);
+    const float bfx = fmaf(fabsf(Ux), g, fmaf(px, r.inv_d.x, r.cf.x) - Ux);
+    const float bfy = fmaf(fabsf(Uy), g, fmaf(py, r.inv_d.y, r.cf.y) - Uy);
+    const float bfz = fmaf(fabsf(Uz), g, fmaf(pz, r.inv_d.z, r.cf.z) - Uz);
+    const bool nx = r.oct & 1u, ny = r.oct & 2u, nz = r.oct & 4u;
+    const uint32_t near_x[2] = {nx ? w3.z : w2.x, nx ? w3.w : w2.y}, far_x[2] = {nx ? w2.x : w3.z, nx ? w2.y : w3.w};
+    const uint32_t near_y[2] = {ny ? w4.x : w2.z, ny ? w4.y : w2.w}, far_y[2] = {ny ? w2.z : w4.x, ny ? w2.w : w4.y};
+    const uint32_t near_z[2] = {nz ? w4.z : w3.x, nz ? w4.w : w3.y}, far_z[2] = {nz ? w3.x : w4.z, nz ? w3.y : w4.w};
+    uint32_t hits = 0;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        int h = c >> 2, b = c & 3;
-        uint32_t m = (meta[h] >> (8 * b)) & 0xffu;
-        bool internal = (imask >> c) & 1u;
-        if (!internal && m == 0u) continue;
-        float lox = __fadd_rn(px, __fmul_rn(ubyte(qlox[h], b), sx));
-        float loy = __fadd_rn(py, __fmul_rn(ubyte(qloy[h], b), sy));
-        float loz = __fadd_rn(pz, __fmul_rn(ubyte(qloz[h], b), sz));
-        float hix = __fadd_rn(px, __fmul_rn(ubyte(qhix[h], b), sx));
-        float hiy = __fadd_rn(py, __fmul_rn(ubyte(qhiy[h], b), sy));
-        float hiz = __fadd_rn(pz, __fmul_rn(ubyte(qhiz[h], b), sz));
-        float t0x = (lox - r.o.x) * r.inv_d.x, t1x = (hix - r.o.x) * r.inv_d.x;
-        float t0y = (loy - r.o.y) * r.inv_d.y, t1y = (hiy - r.o.y) * r.inv_d.y;
-        float t0z = (loz - r.o.z) * r.inv_d.z, t1z = (hiz - r.o.z) * r.inv_d.z;
-        float tn = fmaxf(fmaxf(fminf(t0x, t1x), fminf(t0y, t1y)), fmaxf(fminf(t0z, t1z), 0.0f));
-        float tf = fminf(fminf(fmaxf(t0x, t1x), fmaxf(t0y, t1y)), fminf(fmaxf(t0z, t1z), tmax));
-        if (tn <= tf * kBoxSlack) {
-            if (internal) {
-                ihits |= 1u << (24u + (static_cast<uint32_t>(c) ^ r.oct));
-            } else {
-                uint32_t count_bits = m >> 5;
-                uint32_t offset = m & 31u;
-                thits |= count_bits << offset;
-            }
-        }
+    for (uint32_t c = 0; c < 8; ++c) {
+        const uint32_t h = c >> 2, b = c & 3u;
+        const float tn = fmaxf(max3(fmaf(ubyte_biased(near_x[h], b), Ux, bnx), fmaf(ubyte_biased(near_y[h], b), Uy, bny),
+                                    fmaf(ubyte_biased(near_z[h], b), Uz, bnz)), 0.0f);
+        const float tf = fminf(min3(fmaf(ubyte_biased(far_x[h], b), Ux, bfx), fmaf(ubyte_biased(far_y[h], b), Uy, bfy),
+                                    fmaf(ubyte_biased(far_z[h], b), Uz, bfz)), tmax);
+        if (tn <= tf) hits |= 1u << c;
     }
-    node_group = make_uint2(w1.x, ihits | imask);
+    // Internal children in traversal order: bit c moves to c ^ oct.
+    uint32_t ihits = hits & imask;
+    if (nx) ihits = ((ihits << 1) & 0xaau) | ((ihits >> 1) & 0x55u);
+    if (ny) ihits = ((ihits << 2) & 0xccu) | ((ihits >> 2) & 0x33u);
+    if (nz) ihits = ((ihits << 4) & 0xf0u) | (ihits >> 4);
+    // Leaf children: their triangles (most nodes have few or none hit).
+    uint32_t lhits = hits & ~imask, thits = 0;
+    while (lhits) {
+        const uint32_t c = __ffs(lhits) - 1u;
+        lhits &= lhits - 1u;
+        const uint32_t m = __byte_perm(w1.z, w1.w, c) & 0xffu;
+        thits |= (m >> 5) << (m & 31u);
+    }
+    node_group = make_uint2(w1.x, (ihits << 24) | imask);
     tri_group = make_uint2(w1.y, thits);
 }
 
@@ -515,6 +568,13 @@ __device__ __forceinline__ f3 xf_vector(const float4 &r0, const float4 &r1, cons
             __fadd_rn(__fadd_rn(__fmul_rn(r2.x, v.x), __fmul_rn(r2.y, v.y)), __fmul_rn(r2.z, v.z))};
 }
 
+// The largest coordinate magnitudes of the boxes below a node: its grid's.
+VS_HD f3 node_bound(const uint4 &w0) {
+    return {fabsf(bits_float(w0.x)) + 256.0f * bits_float((w0.w & 0xffu) << 23),
+            fabsf(bits_float(w0.y)) + 256.0f * bits_float(((w0.w >> 8) & 0xffu) << 23),
+            fabsf(bits_float(w0.z)) + 256.0f * bits_float(((w0.w >> 16) & 0xffu) << 23)};
+}
+
 // The closest hit inside instance `inst` with t below the current best.
 static __device__ __noinline__ void instance_closest(const DeviceScene &s, const RayPre &rw, uint32_t inst,
                                                       float tmax, float &best_t, float &best_err, uint32_t &best_prim,
@@ -522,7 +582,8 @@ static __device__ __noinline__ void instance_closest(const DeviceScene &s, const
     const float4 *x = s.inst_xf + 4u * inst;
     const float4 r0 = __ldg(x), r1 = __ldg(x + 1), r2 = __ldg(x + 2), meta = __ldg(x + 3);
     const uint32_t first = __float_as_uint(meta.y);
-    const RayPre r = precompute_ray(xf_point(r0, r1, r2, rw.o), xf_vector(r0, r1, r2, rw.d));
+    const RayPre r = precompute_ray(xf_point(r0, r1, r2, rw.wo), xf_vector(r0, r1, r2, rw.wd),
+                                    node_bound(__ldg(s.nodes + 5u * static_cast<size_t>(__float_as_uint(meta.x)))));
     uint2 stack[kStackSize];
     int sp = 0;
     uint2 ng = make_uint2(__float_as_uint(meta.x), (1u << (24u + (0u ^ r.oct))) | 1u);
@@ -564,7 +625,8 @@ static __device__ __noinline__ bool instance_any(const DeviceScene &s, const Ray
                                                  uint32_t &visits) {
     const float4 *x = s.inst_xf + 4u * inst;
     const float4 r0 = __ldg(x), r1 = __ldg(x + 1), r2 = __ldg(x + 2), meta = __ldg(x + 3);
-    const RayPre r = precompute_ray(xf_point(r0, r1, r2, rw.o), xf_vector(r0, r1, r2, rw.d));
+    const RayPre r = precompute_ray(xf_point(r0, r1, r2, rw.wo), xf_vector(r0, r1, r2, rw.wd),
+                                    node_bound(__ldg(s.nodes + 5u * static_cast<size_t>(__float_as_uint(meta.x)))));
     uint2 stack[kStackSize];
     int sp = 0;
     uint2 ng = make_uint2(__float_as_uint(meta.x), (1u << (24u + (0u ^ r.oct))) | 1u);
@@ -740,6 +802,14 @@ __device__ __forceinline__ void trav_init(TravState &t, const RayPre &r, float t
 // scene pick their instantiation on the host, so the flat traversal keeps its
 // registers.
 constexpr int kLevelsFlat = 0, kLevelsTwo = 1, kLevelsAny = 2;
+
+// Resident blocks of 128 threads per SM asked of the flat traversal kernels:
+// 64 registers a thread.  Left alone the compiler takes 96 to 128 of them for
+// the unrolled child test, and with 4 or 5 blocks the passes take 20 % longer
+// (2.1 M camera rays, 2.3 M triangles: 0.50 ms; 8 blocks 0.41, 9 blocks 0.43,
+// 10 blocks 0.47).
+constexpr int kTraverseBlocks = 8;
+constexpr int traverse_blocks(int levels) { return levels == kLevelsFlat ? kTraverseBlocks : 1; }
 
 // One step of the closest-hit traversal; true when the traversal has ended
 // (the result is in t.best_*).

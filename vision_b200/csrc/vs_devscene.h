@@ -9,6 +9,7 @@ namespace vs {
 // Everything a render kernel reads, passed by value as a kernel parameter.
 struct DeviceScene {
     const uint4 *nodes;          // Bvh8Node array (5 uint4 per node)
+    f3 bound;                    // largest coordinate magnitude of the BVH's boxes, per axis
     const float4 *tri_v;         // leaf-ordered triangles: 3 float4 each, w0 = prim id bits
     const float4 *vtx;           // 2 float4 per vertex: (pos.xyz, u), (normal.xyz, v)
     const uint4 *prims;          // per primitive: vertex indices i, j, k and instance id

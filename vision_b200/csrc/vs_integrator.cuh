@@ -428,7 +428,7 @@ __device__ __forceinline__ bool path_shade_acc(const DeviceScene &s, PathState<N
     LightSample<N> ls = sample_light<N>(s, it, u_light, u_surf, ps.wl);
     Ray sh = spawn_ray_to(it.pos, it.ng, ls.p_light);
     bool occluded = false;
-    if (kTraceShadow) occluded = trace_any(s, precompute_ray(sh.o, sh.d), sh.tmax);
+    if (kTraceShadow) occluded = trace_any(s, precompute_ray(sh.o, sh.d, s.bound), sh.tmax);
     // Material evaluation + BSDF sample (direct_lighting, integrator.cpp:20-44).
     Material mat = s.materials[it.mat];
     const typename ShadeBsdf<N, M>::type bsdf = ShadeBsdf<N, M>::make(s, mat, it.shading, it.ng, it.wo, it.uv, ps.wl);
@@ -480,7 +480,7 @@ __device__ __forceinline__ bool path_shade(const DeviceScene &s, PathState<N> &p
 // One iteration of the bounce loop: closest hit, shading, shadow ray.
 template <int N>
 __device__ __forceinline__ bool path_bounce(const DeviceScene &s, PathState<N> &ps, Interaction *first) {
-    RayPre rp = precompute_ray(ps.ro, ps.rd);
+    RayPre rp = precompute_ray(ps.ro, ps.rd, s.bound);
     Hit hit;
     float t_hit;
     const bool hit_any = trace_closest(s, rp, 3.402823466e+38f, hit, t_hit);

@@ -169,7 +169,7 @@ __device__ __forceinline__ void extend(const Scenes &scenes, const WfBuffers &b,
                 slot = q[i];
                 const float4 o = b.o[slot], d = b.d[slot];
                 s = &scenes(b.st[slot].w);
-                r = precompute_ray(make3(o.x, o.y, o.z), make3(d.x, d.y, d.z));
+                r = precompute_ray(make3(o.x, o.y, o.z), make3(d.x, d.y, d.z), s->bound);
                 trav_init(t, r, 3.402823466e+38f);
                 active = true;
             }
@@ -249,7 +249,7 @@ __device__ __forceinline__ void shadow(const Scenes &scenes, const WfBuffers &b,
                 i = b.sh_perm ? b.sh_perm[k] : k;
                 const float4 o = b.sh_o[i], d = b.sh_d[i];
                 s = &scenes(__float_as_uint(b.sh_c[i].w));
-                r = precompute_ray(make3(o.x, o.y, o.z), make3(d.x, d.y, d.z));
+                r = precompute_ray(make3(o.x, o.y, o.z), make3(d.x, d.y, d.z), s->bound);
                 trav_init(t, r, o.w);
                 active = true;
             }

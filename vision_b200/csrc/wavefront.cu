@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(128) k_wf_generate(const __grid_constant__ Dev
 
 // L: kLevelsFlat or kLevelsTwo, picked on the host from the scene.
 template <int L>
-__global__ void __launch_bounds__(128) k_wf_extend(const __grid_constant__ DeviceScene s,
+__global__ void __launch_bounds__(128, traverse_blocks(L)) k_wf_extend(const __grid_constant__ DeviceScene s,
                                                    const __grid_constant__ WfBuffers b, uint32_t cur) {
     wf::extend<L>(OneScene{&s}, b, cur);
 }
@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(128) k_wf_shade(const __grid_constant__ Device
 }
 
 template <int L>
-__global__ void __launch_bounds__(128) k_wf_shadow(const __grid_constant__ DeviceScene s,
+__global__ void __launch_bounds__(128, traverse_blocks(L)) k_wf_shadow(const __grid_constant__ DeviceScene s,
                                                    const __grid_constant__ WfBuffers b, uint64_t base,
                                                    float4 *radiance) {
     wf::shadow<L>(OneScene{&s}, b, base, radiance);
