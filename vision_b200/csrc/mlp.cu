@@ -5,14 +5,16 @@
 // shared memory and the FP32 accumulator in tensor memory:
 //   inference  (k_mlp_infer): one CTA per SM holding the forward weights once
 //     and running kInferGroups independent 4-warp pipelines, each with its
-//     own 64 tensor-memory columns and two tile buffers; while a pipeline runs
-//     the five layers of one 128-row tile, the TMA engine loads its next tile
-//     into the other buffer (128-byte swizzle, rows past n zero-filled).
-//     M=128 x N=64 (N=16 for the padded output layer), K=64 as four K=16
-//     steps.  Thread t of a pipeline owns tile row t: after each layer it
-//     reads its accumulator row with tcgen05.ld (32x32b), applies ReLU, rounds
-//     to BF16 and writes the next layer's operand row in the no-swizzle
-//     layout, over the consumed feature tile.
+//     own 96 tensor-memory columns (64 of accumulator, 32 of activations) and
+//     two tile buffers; while a pipeline runs the five layers of one 128-row
+//     tile, the TMA engine loads its next tile into the other buffer (128-byte
+//     swizzle, rows past n zero-filled).  M=128 x N=64 (N=16 for the padded
+//     output layer), K=64 as four K=16 steps.  Thread t of a pipeline owns
+//     tile row t: after each layer it reads its accumulator row with
+//     tcgen05.ld (32x32b), rounds to BF16, applies ReLU and writes the next
+//     layer's operand row back to tensor memory with tcgen05.st (two BF16 per
+//     column), where the MMA reads it; only the features and the weights come
+//     from shared memory.
 //   training   (k_mlp_train): the same forward pass keeping every layer's
 //     BF16 input; the relative-L2 loss gradient; the backward data products
 //     dX = dZ W^T (M=128) masked by ReLU'; and the weight gradients
@@ -67,6 +69,15 @@ __device__ __forceinline__ void mma(uint32_t d_tmem, uint64_t a, uint64_t b, uin
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
         "l"(a), "l"(b), "r"(id), "r"(accumulate));
+}
+
+// The same with the A operand in tensor memory (M = 128: lane = row, two K
+// elements per 32-bit column).
+__device__ __forceinline__ void mma_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t id, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b), "r"(id), "r"(accumulate));
 }
 
 __device__ __forceinline__ void commit(uint32_t mbar) {
@@ -128,9 +139,38 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, float *v) {
     for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// The first 4 accumulator columns of this thread's row.
+__device__ __forceinline__ float4 tmem_ld4(uint32_t taddr) {
+    uint32_t r[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    return make_float4(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]), __uint_as_float(r[3]));
+}
+
+// Stores 32 columns of this thread's row and waits for the store.
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t *r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
+        "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+        "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+        "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
     __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<uint32_t *>(&h);
+}
+// ReLU of a pair after rounding (the same value as rounding the ReLU; NaN
+// gives 0 either way).
+__device__ __forceinline__ uint32_t pack2_relu(float a, float b) {
+    const __nv_bfloat162 h = __hmax2(__floats2bfloat162_rn(a, b), __nv_bfloat162(__ushort_as_bfloat16(0), __ushort_as_bfloat16(0)));
+    return *reinterpret_cast<const uint32_t *>(&h);
 }
 __device__ __forceinline__ float bf_lo(uint32_t u) { return __uint_as_float(u << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t u) { return __uint_as_float(u & 0xFFFF0000u); }
@@ -253,7 +293,15 @@ __device__ __forceinline__ bool group_sync_and(uint32_t g, bool v) {
     return r != 0u;
 }
 
+// Five pipelines of 96 columns fill the 512 of tensor memory.  With the
+// activations in shared memory instead (written by the epilogue, read by the
+// next MMA) each tile moved 200 KB through shared memory, 1600 of the 2300
+// cycles it took; here it moves 66 KB.
+// 2,073,600 rows: 130 -> 106 us (bound now by the epilogues' latency and the
+// conversions: ALU 51 %, tensor pipe 33 %, 2.7 TB/s).
 constexpr uint32_t kInferGroups = 5;
+constexpr uint32_t kInferCols = 96;
+static_assert(kInferGroups * kInferCols <= 512u, "tensor memory columns");
 constexpr uint32_t kInferThreads = 128u * kInferGroups;
 constexpr uint32_t kInferBars = 3u * kInferGroups;  // per pipeline: two tile loads, one MMA
 constexpr uint32_t kInferSmem = 1024u + kPackFwdBytes + kInferGroups * 2u * kTileBytes + 8u * kInferBars + 16u;
@@ -281,13 +329,13 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(const __grid_con
     fence_before();
     __syncthreads();
     fence_after();
-    // Pipeline g: accumulator columns [64 g, 64 g + 64), tile buffers
-    // buf0 + {0, kTileBytes}, barriers load[0], load[1], mma.
-    const uint32_t tmem = *slot + 64u * g;
+    // Pipeline g: accumulator columns [96 g, 96 g + 64), activation columns
+    // [96 g + 64, 96 g + 96), tile buffers buf0 + {0, kTileBytes}, barriers
+    // load[0], load[1], mma.
+    const uint32_t tmem = *slot + kInferCols * g, act = tmem + 64u;
     const uint32_t lane = (gt & ~31u) << 16;
     const uint32_t wbase = smem_u32(w);
-    uint8_t *tile0 = bufs + g * 2u * kTileBytes;
-    const uint32_t buf0 = smem_u32(tile0);
+    const uint32_t buf0 = smem_u32(bufs + g * 2u * kTileBytes);
     const uint32_t mb_load = smem_u32(bars + 3u * g), mb_mma = mb_load + 16u;
     const uint32_t tiles = (n + kTile - 1) / kTile;
     const uint32_t stride = gridDim.x * kInferGroups;
@@ -303,7 +351,6 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(const __grid_con
     for (uint32_t k = 0; tt < tiles && ok; tt += stride, ++k) {
         const uint32_t cur = k & 1u, nxt = cur ^ 1u;
         const uint32_t buf = buf0 + cur * kTileBytes;
-        uint8_t *tile = tile0 + cur * kTileBytes;
         // The other buffer held the previous tile, whose last MMA has
         // completed: load the next tile into it now.
         if (tt + stride < tiles) {
@@ -323,10 +370,13 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(const __grid_con
         for (int l = 0; l < 5; ++l) {
             if (gt == 0) {
                 const uint32_t id = l < 4 ? idesc(128, 64, 0, 0) : idesc(128, 16, 0, 0);
+                if (l == 0) {
 #pragma unroll
-                for (int s = 0; s < 4; ++s)
-                    mma(tmem, l == 0 ? tile_sw128_desc(buf, s) : tile_kdesc(buf, s), w_fwd_desc(wbase, l, s), id,
-                        s > 0);
+                    for (int s = 0; s < 4; ++s) mma(tmem, tile_sw128_desc(buf, s), w_fwd_desc(wbase, 0, s), id, s > 0);
+                } else {
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) mma_ta(tmem, act + 8u * s, w_fwd_desc(wbase, l, s), id, s > 0);
+                }
                 commit(mb_mma);
             }
             done = mbar_wait(mb_mma, ph_mma);
@@ -337,14 +387,13 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(const __grid_con
             if (done && l < 4) {
                 float v[64];
                 tmem_ld64(tmem + lane, v);
+                uint32_t h[32];
 #pragma unroll
-                for (int i = 0; i < 64; ++i) v[i] = fmaxf(v[i], 0.0f);
-                st_row64(tile, gt, v);
-                fence_async_smem();
+                for (int i = 0; i < 32; ++i) h[i] = pack2_relu(v[2 * i], v[2 * i + 1]);
+                tmem_st32(act + lane, h);
             } else if (done) {
-                float v[16];
-                tmem_ld16(tmem + lane, v);
-                if (row < n) out[row] = make_float4(v[0], v[1], v[2], 0.0f);
+                const float4 v = tmem_ld4(tmem + lane);
+                if (row < n) out[row] = make_float4(v.x, v.y, v.z, 0.0f);
             }
             fence_before();
             ok = group_sync_and(g, done);
