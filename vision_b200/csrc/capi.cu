@@ -1593,7 +1593,6 @@ struct vs_cache {
         cudaFree(st.m);
         cudaFree(st.v);
         cudaFree(st.grad);
-        cudaFree(st.loss);
         cudaFree(st.err);
     }
 };
@@ -1622,14 +1621,13 @@ int vs_cache_create(vs_context *ctx, uint64_t seed, vs_cache **out) {
     if (e == cudaSuccess) e = cudaMalloc(&s.pack, sizeof(uint16_t) * kMlpPackElems);
     if (e == cudaSuccess) e = cudaMalloc(&s.m, sizeof(float) * kMlpParams);
     if (e == cudaSuccess) e = cudaMalloc(&s.v, sizeof(float) * kMlpParams);
-    if (e == cudaSuccess) e = cudaMalloc(&s.grad, sizeof(float) * kMlpParams);
-    if (e == cudaSuccess) e = cudaMalloc(&s.loss, sizeof(double));
+    if (e == cudaSuccess) e = cudaMalloc(&s.grad, kMlpGradBytes);
+    if (e == cudaSuccess) s.loss = reinterpret_cast<double *>(s.grad + kMlpParams);
     if (e == cudaSuccess) e = cudaMalloc(&s.err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(s.pack, 0, sizeof(uint16_t) * kMlpPackElems);
     if (e == cudaSuccess) e = cudaMemset(s.m, 0, sizeof(float) * kMlpParams);
     if (e == cudaSuccess) e = cudaMemset(s.v, 0, sizeof(float) * kMlpParams);
-    if (e == cudaSuccess) e = cudaMemset(s.grad, 0, sizeof(float) * kMlpParams);
-    if (e == cudaSuccess) e = cudaMemset(s.loss, 0, sizeof(double));
+    if (e == cudaSuccess) e = cudaMemset(s.grad, 0, kMlpGradBytes);
     if (e == cudaSuccess) e = cudaMemset(s.err, 0, sizeof(int));
     if (e != cudaSuccess) {
         delete c;

@@ -16,13 +16,13 @@
 //     column), where the MMA reads it; only the features and the weights come
 //     from shared memory.
 //   training   (k_mlp_train): the same forward pass keeping every layer's
-//     BF16 input; the relative-L2 loss gradient; the backward data products
-//     dX = dZ W^T (M=128) masked by ReLU'; and the weight gradients
-//     dW = X^T dZ as M=64 MMAs whose operands are the same shared-memory
-//     tiles read MN-major, accumulated in tensor memory over all tiles of the
-//     CTA and added to the global FP32 gradient once per CTA.
+//     BF16 input in shared memory; the relative-L2 loss gradient; the backward
+//     data products dX = dZ W^T (M=128) masked by ReLU'; and the weight
+//     gradients dW = X^T dZ as M=64 MMAs whose operands are the same
+//     shared-memory tiles read MN-major, accumulated in tensor memory over all
+//     tiles of the CTA and added to the global FP32 gradient once per CTA.
 //   k_mlp_adam updates the FP32 master weights; k_mlp_pack rewrites the BF16
-//   operand images (forward: W as [out][in]; backward: W as [in][out]).
+//   operand image (W as [out][in], read MN-major for the data gradients).
 // Shared-memory operands use the canonical no-swizzle layout: 8-row x 16-byte
 // core matrices, rows of a core matrix 16 B apart; for a K-major operand with
 // R rows, core matrices along M/N are 128 B apart (SBO) and along K R*16 B
@@ -44,7 +44,7 @@ namespace {
 
 constexpr int kTile = 128;
 constexpr uint32_t kTileBytes = kTile * 64 * 2;       // 16 KB activation tile
-constexpr uint32_t kPackFwdBytes = kMlpPackFwd * 2;   // 34,816 B
+constexpr uint32_t kPackBytes = kMlpPackElems * 2;     // 34,816 B
 constexpr long long kWaitCycles = 4000000000ll;       // ~2 s at 1.9 GHz
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -109,18 +109,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
     }
 }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
 // Issues the loads of 64 accumulator columns (four 32x32b.x16) and waits for
 // them once.
 __device__ __forceinline__ void tmem_ld64(uint32_t taddr, float *v) {
@@ -181,13 +169,6 @@ __device__ __forceinline__ uint32_t tile_chunk(uint32_t r, uint32_t kc) {
     return kc * 2048u + (r >> 3) * 128u + (r & 7u) * 16u;
 }
 
-// Reads the 64 accumulator columns [col, col + 64) of this thread's row.
-__device__ __forceinline__ void ld_row64(uint32_t tmem, uint32_t col, float *v) {
-    uint32_t lane = (threadIdx.x & ~31u) << 16;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) tmem_ld16(tmem + lane + col + 16u * q, v + 16 * q);
-}
-
 // Writes 64 values as BF16 into row r of a 128-row tile.
 __device__ __forceinline__ void st_row64(uint8_t *tile, uint32_t r, const float *v) {
 #pragma unroll
@@ -213,15 +194,11 @@ __device__ __forceinline__ void ld_row64_bf(const uint8_t *tile, uint32_t r, flo
     }
 }
 
-// Loads row `row` of the global feature matrix (zeros past n) into tile row r.
-__device__ __forceinline__ void load_features(uint8_t *tile, uint32_t r, const uint16_t *feat, uint64_t row,
-                                              uint32_t n) {
+// Row `row` of the global feature matrix (zeros past n).
+__device__ __forceinline__ void ld_features(uint4 *f, const uint16_t *feat, uint64_t row, uint32_t n) {
     const uint4 *src = reinterpret_cast<const uint4 *>(feat + row * 64u);
 #pragma unroll
-    for (int kc = 0; kc < 8; ++kc) {
-        uint4 u = row < n ? __ldg(src + kc) : make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4 *>(tile + tile_chunk(r, kc)) = u;
-    }
+    for (int kc = 0; kc < 8; ++kc) f[kc] = row < n ? __ldg(src + kc) : make_uint4(0, 0, 0, 0);
 }
 
 __device__ __forceinline__ void copy_to_smem(uint8_t *dst, const uint4 *src, uint32_t bytes) {
@@ -234,11 +211,12 @@ __device__ __forceinline__ uint64_t w_fwd_desc(uint32_t wbase, int l, int s) {
     if (l < 4) return sdesc(wbase + l * 8192u + s * 2048u, 1024u, 128u);
     return sdesc(wbase + 4u * 8192u + s * 512u, 256u, 128u);
 }
-// Backward weight descriptors: layer l < 4 is [64 in][64 out] (LBO 1024);
-// the output layer [64 in][16 out], one K step.
+// The same image read for dX = dZ W^T: N = in, K = out, MN-major (the next 8
+// out rows 128 B on, the next 8 in columns 1024 B or, in the output layer's
+// image, 256 B on); K step s advances 16 out rows.
 __device__ __forceinline__ uint64_t w_bwd_desc(uint32_t wbase, int l, int s) {
-    if (l < 4) return sdesc(wbase + l * 8192u + s * 2048u, 1024u, 128u);
-    return sdesc(wbase + 4u * 8192u, 1024u, 128u);
+    if (l < 4) return sdesc(wbase + l * 8192u + s * 256u, 128u, 1024u);
+    return sdesc(wbase + 4u * 8192u, 128u, 256u);
 }
 // A 128-row activation tile as a K-major operand, K step s.
 __device__ __forceinline__ uint64_t tile_kdesc(uint32_t base, int s) { return sdesc(base + s * 4096u, 2048u, 128u); }
@@ -304,7 +282,7 @@ constexpr uint32_t kInferCols = 96;
 static_assert(kInferGroups * kInferCols <= 512u, "tensor memory columns");
 constexpr uint32_t kInferThreads = 128u * kInferGroups;
 constexpr uint32_t kInferBars = 3u * kInferGroups;  // per pipeline: two tile loads, one MMA
-constexpr uint32_t kInferSmem = 1024u + kPackFwdBytes + kInferGroups * 2u * kTileBytes + 8u * kInferBars + 16u;
+constexpr uint32_t kInferSmem = 1024u + kPackBytes + kInferGroups * 2u * kTileBytes + 8u * kInferBars + 16u;
 static_assert(kInferSmem <= 232448u, "inference shared memory above the per-CTA limit");
 
 __global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(const __grid_constant__ CUtensorMap fmap, uint32_t n,
@@ -315,7 +293,7 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(const __grid_con
     const uint32_t raw = smem_u32(smem_raw);
     uint8_t *smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     uint8_t *w = smem;
-    uint8_t *bufs = smem + kPackFwdBytes;
+    uint8_t *bufs = smem + kPackBytes;
     uint64_t *bars = reinterpret_cast<uint64_t *>(bufs + kInferGroups * 2u * kTileBytes);
     uint32_t *slot = reinterpret_cast<uint32_t *>(bars + kInferBars);
     const uint32_t tid = threadIdx.x, g = tid >> 7, gt = tid & 127u;
@@ -324,7 +302,7 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(const __grid_con
         for (uint32_t i = 0; i < kInferBars; ++i) mbar_init(smem_u32(bars + i), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    copy_to_smem(w, wpack, kPackFwdBytes);
+    copy_to_smem(w, wpack, kPackBytes);
     fence_async_smem();
     fence_before();
     __syncthreads();
@@ -412,196 +390,232 @@ __global__ void __launch_bounds__(kInferThreads, 1) k_mlp_infer(const __grid_con
     if (tid < 32) tmem_free(*slot, 512);
 }
 
-// Training shared memory: forward and backward weight images, the input tile
-// X0, hidden activations H1..H4, the gradient tile G, the output-gradient
-// tile DO (128 x 16), barrier and slots.
-constexpr uint32_t kOffWf = 0;
-constexpr uint32_t kOffWb = kPackFwdBytes;
-constexpr uint32_t kOffX = 2 * kPackFwdBytes;
-constexpr uint32_t kOffG = kOffX + 5 * kTileBytes;
-constexpr uint32_t kOffDO = kOffG + kTileBytes;
-constexpr uint32_t kOffBar = kOffDO + 4096;
-constexpr uint32_t kTrainSmem = kOffBar + 64;
-constexpr uint32_t kTrainCols = 512;   // D: 0..63; dW0..dW3: 64 + 64 l; dW4: 320..335
+// Training shared memory: the weight image, then per pipeline the input tile X0
+// and the hidden activations H1..H4 and the output-gradient tile DO
+// (128 x 16); barriers and slots.
+constexpr uint32_t kTrainPipes = 2;
+constexpr uint32_t kTrainThreads = 128u * kTrainPipes + 32u;
+constexpr uint32_t kTrainPipeBytes = 5u * kTileBytes + 4096u;
+constexpr uint32_t kOffPipe = kPackBytes;
+constexpr uint32_t kOffBar = kOffPipe + kTrainPipes * kTrainPipeBytes;
+constexpr uint32_t kTrainSmem = kOffBar + 128u;
+constexpr uint32_t kTrainCols = 512;   // D of pipeline p: 64 p; dW0..dW3: 128 + 64 l; dW4: 384..399
+static_assert(kTrainSmem <= 232448u, "training shared memory above the per-CTA limit");
 
-__global__ void __launch_bounds__(128, 1) k_mlp_train(const uint16_t *__restrict__ feat,
-                                                      const float4 *__restrict__ target, uint32_t n,
-                                                      const uint4 *__restrict__ wpack, float loss_scale,
-                                                      float *__restrict__ grad, double *loss, int *err) {
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
+}
+
+// Adds four consecutive floats (16-byte aligned) to global memory.
+__device__ __forceinline__ void red_add4(float *p, const float *v) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+                 "f"(v[3])
+                 : "memory");
+}
+
+// The forward pass, the loss gradient and the backward pass of one tile are
+// ten dependent rounds of an MMA batch and an epilogue, each mostly latency.
+// Two pipelines of 128 threads (one tile each) alternate, so one's epilogue
+// runs under the other's MMAs, and a 65,536-sample step needs two passes over
+// the tiles instead of four.  A ninth warp issues every MMA, in a fixed order,
+// because both pipelines accumulate the weight gradients in the same columns.
+// To fit two pipelines, a layer's gradient dZ overwrites the activations it
+// was masked with, and the data gradient reads the forward weight image
+// MN-major instead of a second, transposed copy.
+// 65,536 samples: kernel 71 -> 34 us; four steps with their updates 424 -> 269 us.
+__global__ void __launch_bounds__(kTrainThreads, 1) k_mlp_train(const uint16_t *__restrict__ feat,
+                                                                const float4 *__restrict__ target, uint32_t n,
+                                                                const uint4 *__restrict__ wpack, float loss_scale,
+                                                                float *__restrict__ grad, double *loss, int *err) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t *act[5];
-#pragma unroll
-    for (int l = 0; l < 5; ++l) act[l] = smem + kOffX + l * kTileBytes;  // X0, H1, H2, H3, H4
-    uint8_t *G = smem + kOffG;
-    uint8_t *DO = smem + kOffDO;
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + kOffBar);
-    uint32_t *slot = reinterpret_cast<uint32_t *>(smem + kOffBar + 8);
-    float *red = reinterpret_cast<float *>(smem + kOffBar + 16);
-    const uint32_t tid = threadIdx.x;
-    const uint32_t mbar_s = smem_u32(mbar);
+    // Barriers: ready[p] (the pipeline's 128 threads have written their
+    // operands), done[p] (its MMA batch has completed).
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kOffBar);
+    uint32_t *slot = reinterpret_cast<uint32_t *>(smem + kOffBar + 32);
+    float *red = reinterpret_cast<float *>(smem + kOffBar + 48);
+    const uint32_t tid = threadIdx.x, pipe = tid >> 7, gt = tid & 127u;
     if (tid < 32) tmem_alloc(smem_u32(slot), kTrainCols);
     if (tid == 0) {
-        mbar_init(mbar_s, 1);
+        for (uint32_t p = 0; p < kTrainPipes; ++p) {
+            mbar_init(smem_u32(bars + p), 128);
+            mbar_init(smem_u32(bars + kTrainPipes + p), 1);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    copy_to_smem(smem + kOffWf, wpack, 2 * kPackFwdBytes);
+    copy_to_smem(smem, wpack, kPackBytes);
     fence_async_smem();
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem = *slot;
-    const uint32_t wf = smem_u32(smem + kOffWf), wb = smem_u32(smem + kOffWb);
-    uint32_t abase[5];
-#pragma unroll
-    for (int l = 0; l < 5; ++l) abase[l] = smem_u32(act[l]);
-    const uint32_t gbase = smem_u32(G), dobase = smem_u32(DO);
-    const uint32_t lane = (tid & ~31u) << 16;
-    uint32_t phase = 0;
-    bool ok = true;
-    bool first = true;
-    float loss_acc = 0.0f;
+    const uint32_t wb = smem_u32(smem);
     const uint32_t tiles = (n + kTile - 1) / kTile;
-    auto sync_all = [&]() {
-        fence_before();
-        __syncthreads();
-        fence_after();
-    };
-    auto wait_mma = [&]() {
-        const bool done = ok && mbar_wait(mbar_s, phase);
-        phase ^= 1u;
-        ok = __syncthreads_and(done) != 0;
-        fence_after();
-    };
-    for (uint32_t tt = blockIdx.x; tt < tiles && ok; tt += gridDim.x) {
-        const uint64_t row = static_cast<uint64_t>(tt) * kTile + tid;
-        const bool valid = row < n;
-        load_features(act[0], tid, feat, row, n);
-        fence_async_smem();
-        sync_all();
-        // Forward: layers 0..3 into H1..H4, output layer into registers.
-        float y[3] = {0.0f, 0.0f, 0.0f};
-        for (int l = 0; l < 5 && ok; ++l) {
-            if (tid == 0) {
-                const uint32_t id = l < 4 ? idesc(128, 64, 0, 0) : idesc(128, 16, 0, 0);
+    const uint32_t stride = gridDim.x * kTrainPipes;
+    bool ok = true;
+    float loss_acc = 0.0f;
+    if (pipe == kTrainPipes) {
+        // The issuing thread: rounds of both pipelines in turn (0..4: forward
+        // layers, 5..9: backward layers 4..0).
+        if (gt == 0) {
+            uint32_t phase[kTrainPipes] = {0u, 0u};
+            for (uint32_t base = blockIdx.x; base < tiles && ok; base += stride) {
+                for (int round = 0; round < 10 && ok; ++round) {
 #pragma unroll
-                for (int s = 0; s < 4; ++s) mma(tmem, tile_kdesc(abase[l], s), w_fwd_desc(wf, l, s), id, s > 0);
-                commit(mbar_s);
-            }
-            wait_mma();
-            if (!ok) break;
-            if (l < 4) {
-                float v[64];
-                ld_row64(tmem, 0, v);
+                    for (uint32_t p = 0; p < kTrainPipes; ++p) {
+                        if (!ok || base + p * gridDim.x >= tiles) continue;
+                        ok = mbar_wait(smem_u32(bars + p), phase[p]);
+                        if (!ok) continue;
+                        phase[p] ^= 1u;
+                        fence_after();
+                        const uint32_t act = smem_u32(smem + kOffPipe + p * kTrainPipeBytes);
+                        const uint32_t d = tmem + 64u * p;
+                        if (round < 5) {
+                            const uint32_t id = round < 4 ? idesc(128, 64, 0, 0) : idesc(128, 16, 0, 0);
 #pragma unroll
-                for (int i = 0; i < 64; ++i) v[i] = fmaxf(v[i], 0.0f);
-                st_row64(act[l + 1], tid, v);
-                fence_async_smem();
-            } else {
-                float v[16];
-                tmem_ld16(tmem + lane, v);
-                y[0] = v[0];
-                y[1] = v[1];
-                y[2] = v[2];
-            }
-            sync_all();
-        }
-        if (!ok) break;
-        // Relative L2 loss (denominator without gradient) and its gradient.
-        float go[3] = {0.0f, 0.0f, 0.0f};
-        if (valid) {
-            float4 t = target[row];
-            const float tv[3] = {t.x, t.y, t.z};
+                            for (int s = 0; s < 4; ++s)
+                                mma(d, tile_kdesc(act + round * kTileBytes, s), w_fwd_desc(wb, round, s), id, s > 0);
+                        } else {
+                            // dW_l += X_l^T dZ_l, dX_l = dZ_l W_l^T; dZ_l lies in H_{l+1}'s tile (l = 4: DO).
+                            const int l = 9 - round;
+                            const uint32_t x = act + l * kTileBytes, dz = x + kTileBytes;
+                            const uint32_t dw = tmem + 128u + 64u * l;
+                            const uint32_t id_w = l == 4 ? idesc(64, 16, 1, 1) : idesc(64, 64, 1, 1);
+                            const uint32_t first = base == blockIdx.x && p == 0u ? 1u : 0u;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                float e = y[c] - tv[c];
-                float den = y[c] * y[c] + 0.01f;
-                loss_acc += e * e / den;
-                go[c] = 2.0f * e / den * loss_scale;
-            }
-        }
-        {
-            uint4 u0 = make_uint4(pack2(go[0], go[1]), pack2(go[2], 0.0f), 0u, 0u);
-            *reinterpret_cast<uint4 *>(DO + tile_chunk(tid, 0)) = u0;
-            *reinterpret_cast<uint4 *>(DO + tile_chunk(tid, 1)) = make_uint4(0u, 0u, 0u, 0u);
-        }
-        fence_async_smem();
-        sync_all();
-        // Backward, layer by layer: dW_l += X_l^T dZ_l, dX_l = dZ_l W_l^T, dZ_{l-1} = dX_l * (X_l > 0).
-        for (int l = 4; l >= 0 && ok; --l) {
-            if (tid == 0) {
-                const uint32_t dz = l == 4 ? dobase : gbase;
-                const uint32_t dw_col = l == 4 ? 320u : 64u + 64u * l;
-                const uint32_t id_w = l == 4 ? idesc(64, 16, 1, 1) : idesc(64, 64, 1, 1);
+                            for (int s = 0; s < 8; ++s)
+                                mma(dw, tile_mndesc(x, s), tile_mndesc(dz, s), id_w, (!first || s > 0) ? 1u : 0u);
+                            if (l == 4) {
+                                mma(d, sdesc(dz, 2048u, 128u), w_bwd_desc(wb, 4, 0), idesc(128, 64, 0, 1), 0u);
+                            } else if (l > 0) {
 #pragma unroll
-                for (int s = 0; s < 8; ++s)
-                    mma(tmem + dw_col, tile_mndesc(abase[l], s), tile_mndesc(dz, s), id_w, (!first || s > 0) ? 1u : 0u);
-                if (l > 0) {
-                    if (l == 4) {
-                        mma(tmem, sdesc(dobase, 2048u, 128u), w_bwd_desc(wb, 4, 0), idesc(128, 64, 0, 0), 0u);
-                    } else {
-#pragma unroll
-                        for (int s = 0; s < 4; ++s)
-                            mma(tmem, tile_kdesc(gbase, s), w_bwd_desc(wb, l, s), idesc(128, 64, 0, 0), s > 0);
+                                for (int s = 0; s < 4; ++s)
+                                    mma(d, tile_kdesc(dz, s), w_bwd_desc(wb, l, s), idesc(128, 64, 0, 1), s > 0);
+                            }
+                        }
+                        commit(smem_u32(bars + kTrainPipes + p));
                     }
                 }
-                commit(mbar_s);
             }
-            wait_mma();
+        }
+    } else {
+        uint8_t *act = smem + kOffPipe + pipe * kTrainPipeBytes;
+        uint8_t *DO = act + 5u * kTileBytes;
+        const uint32_t ready = smem_u32(bars + pipe), done = smem_u32(bars + kTrainPipes + pipe);
+        const uint32_t lane = (gt & ~31u) << 16;
+        const uint32_t d = tmem + 64u * pipe + lane;
+        uint32_t phase = 0u;
+        // Publishes this thread's operand row and waits for the MMA batch.
+        auto round_trip = [&]() {
+            fence_async_smem();
+            fence_before();
+            mbar_arrive(ready);
+            ok = __all_sync(0xffffffffu, mbar_wait(done, phase)) != 0;
+            phase ^= 1u;
+            fence_after();
+        };
+        uint32_t tt = blockIdx.x + pipe * gridDim.x;
+        uint4 f[8];
+        ld_features(f, feat, static_cast<uint64_t>(tt) * kTile + gt, n);
+        for (; tt < tiles && ok; tt += stride) {
+            const uint64_t row = static_cast<uint64_t>(tt) * kTile + gt;
+            const bool valid = row < n;
+#pragma unroll
+            for (int kc = 0; kc < 8; ++kc) *reinterpret_cast<uint4 *>(act + tile_chunk(gt, kc)) = f[kc];
+            // The next tile's row, in flight under this tile's rounds.
+            ld_features(f, feat, row + static_cast<uint64_t>(stride) * kTile, n);
+            const float4 t = valid ? __ldg(target + row) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            // Forward: layers 0..3 into H1..H4, output layer into registers.
+            for (int l = 0; l < 4 && ok; ++l) {
+                round_trip();
+                if (!ok) break;
+                float v[64];
+                tmem_ld64(d, v);
+#pragma unroll
+                for (int i = 0; i < 64; ++i) v[i] = fmaxf(v[i], 0.0f);
+                st_row64(act + (l + 1) * kTileBytes, gt, v);
+            }
             if (!ok) break;
-            if (l > 0) {
+            round_trip();
+            if (!ok) break;
+            const float4 y4 = tmem_ld4(d);
+            // Relative L2 loss (denominator without gradient) and its gradient.
+            float go[3] = {0.0f, 0.0f, 0.0f};
+            if (valid) {
+                const float y[3] = {y4.x, y4.y, y4.z}, tv[3] = {t.x, t.y, t.z};
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    float e = y[c] - tv[c];
+                    float den = y[c] * y[c] + 0.01f;
+                    loss_acc += e * e / den;
+                    go[c] = 2.0f * e / den * loss_scale;
+                }
+            }
+            *reinterpret_cast<uint4 *>(DO + tile_chunk(gt, 0)) = make_uint4(pack2(go[0], go[1]), pack2(go[2], 0.0f), 0u, 0u);
+            *reinterpret_cast<uint4 *>(DO + tile_chunk(gt, 1)) = make_uint4(0u, 0u, 0u, 0u);
+            // Backward: dZ_{l-1} = dX_l where H_l > 0, written over H_l.
+            for (int l = 4; l > 0 && ok; --l) {
+                round_trip();
+                if (!ok) break;
                 float v[64], h[64];
-                ld_row64(tmem, 0, v);
-                ld_row64_bf(act[l], tid, h);
+                tmem_ld64(d, v);
+                ld_row64_bf(act + l * kTileBytes, gt, h);
 #pragma unroll
                 for (int i = 0; i < 64; ++i) v[i] = h[i] > 0.0f ? v[i] : 0.0f;
-                st_row64(G, tid, v);
-                fence_async_smem();
+                st_row64(act + l * kTileBytes, gt, v);
             }
-            sync_all();
+            if (!ok) break;
+            round_trip();
         }
-        first = false;
     }
+    fence_before();
+    const bool all_ok = __syncthreads_and(ok) != 0;
+    fence_after();
     // Weight gradients: rows of an M=64 accumulator live in lanes 16w..16w+15
-    // of warp w's quarter (row 16w + t in lane 32w + t, t < 16).
-    if (ok && !first) {
-        const uint32_t r = 16u * (tid >> 5) + (tid & 31u);
-        const bool holder = (tid & 31u) < 16u;
-        for (int l = 0; l < 4; ++l) {
+    // of warp w's quarter (row 16w + t in lane 32w + t, t < 16); pipeline p's
+    // warps add layers 2p and 2p + 1, pipeline 0's the output layer too.
+    if (all_ok && pipe < kTrainPipes && blockIdx.x < tiles) {
+        const uint32_t lane = (gt & ~31u) << 16;
+        const uint32_t r = 16u * (gt >> 5) + (gt & 31u);
+        const bool holder = (gt & 31u) < 16u;
+        for (uint32_t l = 2u * pipe; l < 2u * pipe + 2u; ++l) {
             float v[64];
-            ld_row64(tmem, 64u + 64u * l, v);
-            if (holder)
-                for (int c = 0; c < 64; ++c) atomicAdd(grad + l * 4096 + r * 64 + c, v[c]);
+            tmem_ld64(tmem + lane + 128u + 64u * l, v);
+            if (holder) {
+#pragma unroll
+                for (int c = 0; c < 64; c += 4) red_add4(grad + l * 4096u + r * 64u + c, v + c);
+            }
         }
-        float v[16];
-        tmem_ld16(tmem + lane + 320u, v);
-        if (holder)
-            for (int c = 0; c < 3; ++c) atomicAdd(grad + 4 * 4096 + r * 3 + c, v[c]);
+        if (pipe == 0) {
+            const float4 v = tmem_ld4(tmem + lane + 384u);
+            if (holder) {
+                atomicAdd(grad + 4 * 4096 + r * 3, v.x);
+                atomicAdd(grad + 4 * 4096 + r * 3 + 1, v.y);
+                atomicAdd(grad + 4 * 4096 + r * 3 + 2, v.z);
+            }
+        }
     }
     // Loss reduction.
-    for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
-    if ((tid & 31u) == 0) red[tid >> 5] = loss_acc;
+    if (pipe < kTrainPipes) {
+        for (int o = 16; o > 0; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
+        if ((tid & 31u) == 0) red[tid >> 5] = loss_acc;
+    }
     fence_before();
     __syncthreads();
     fence_after();
     if (tid == 0) {
-        double s = static_cast<double>(red[0]) + red[1] + red[2] + red[3];
-        atomicAdd(loss, s * loss_scale);
-        if (!ok) atomicExch(err, 1);
+        double sum = 0.0;
+        for (uint32_t w = 0; w < 4u * kTrainPipes; ++w) sum += static_cast<double>(red[w]);
+        atomicAdd(loss, sum * loss_scale);
+        if (!all_ok) atomicExch(err, 1);
     }
     if (tid < 32) tmem_free(tmem, kTrainCols);
 }
 
-// Packed-image offsets (elements) of weight (l, in, out).
-__device__ __forceinline__ uint32_t off_fwd(int l, uint32_t in, uint32_t out) {
+// Packed-image offset (elements) of weight (l, in, out).
+__device__ __forceinline__ uint32_t pack_offset(int l, uint32_t in, uint32_t out) {
     if (l < 4) return l * 4096u + (in >> 3) * 512u + (out >> 3) * 64u + (out & 7u) * 8u + (in & 7u);
     return 4u * 4096u + (in >> 3) * 128u + (out & 7u) * 8u + (in & 7u);
 }
-__device__ __forceinline__ uint32_t off_bwd(int l, uint32_t in, uint32_t out) {
-    const uint32_t b = static_cast<uint32_t>(kMlpPackFwd);
-    if (l < 4) return b + l * 4096u + (out >> 3) * 512u + (in >> 3) * 64u + (in & 7u) * 8u + (out & 7u);
-    return b + 4u * 4096u + (in >> 3) * 64u + (in & 7u) * 8u + (out & 7u);
-}
-
 __device__ __forceinline__ void param_coords(uint32_t i, int &l, uint32_t &in, uint32_t &out) {
     if (i < 4u * 4096u) {
         l = static_cast<int>(i / 4096u);
@@ -622,8 +636,7 @@ __global__ void k_mlp_pack(const float *w, uint16_t *pack) {
     param_coords(i, l, in, out);
     __nv_bfloat16 h = __float2bfloat16_rn(w[i]);
     uint16_t u = *reinterpret_cast<uint16_t *>(&h);
-    pack[off_fwd(l, in, out)] = u;
-    pack[off_bwd(l, in, out)] = u;
+    pack[pack_offset(l, in, out)] = u;
 }
 
 __global__ void k_mlp_adam(float *w, float *m, float *v, const float *g, MlpAdam a, uint16_t *pack) {
@@ -643,8 +656,7 @@ __global__ void k_mlp_adam(float *w, float *m, float *v, const float *g, MlpAdam
     param_coords(i, l, in, out);
     __nv_bfloat16 h = __float2bfloat16_rn(wi);
     uint16_t u = *reinterpret_cast<uint16_t *>(&h);
-    pack[off_fwd(l, in, out)] = u;
-    pack[off_bwd(l, in, out)] = u;
+    pack[pack_offset(l, in, out)] = u;
 }
 
 int g_sm_count = 0;
@@ -728,8 +740,8 @@ cudaError_t mlp_train_step(const MlpState &s, const uint16_t *feat, const float4
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    cudaError_t e = cudaMemsetAsync(s.grad, 0, sizeof(float) * kMlpParams, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s.loss, 0, sizeof(double), st);
+    // The loss follows the gradient: one clear for both.
+    cudaError_t e = cudaMemsetAsync(s.grad, 0, kMlpGradBytes, st);
     if (e != cudaSuccess) return e;
     if (n > 0) {
         int sms = 0;
@@ -738,7 +750,7 @@ cudaError_t mlp_train_step(const MlpState &s, const uint16_t *feat, const float4
         uint32_t tiles = (n + kTile - 1) / kTile;
         uint32_t grid = static_cast<uint32_t>(sms);
         if (grid > tiles) grid = tiles;
-        k_mlp_train<<<grid, 128, kTrainSmem, st>>>(feat, target, n, reinterpret_cast<const uint4 *>(s.pack),
+        k_mlp_train<<<grid, kTrainThreads, kTrainSmem, st>>>(feat, target, n, reinterpret_cast<const uint4 *>(s.pack),
                                                    adam.loss_scale, s.grad, s.loss, s.err);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;

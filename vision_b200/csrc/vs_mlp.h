@@ -3,6 +3,7 @@
 // tcgen05 tensor cores (mlp.cu).
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -15,10 +16,12 @@ constexpr int kMlpOutPad = 16;     // output layer padded to the smallest M=128 
 constexpr int kMlpHiddenLayers = 4;
 // Weights: 4 x 64 x 64 (input + 3 hidden-to-hidden) + 64 x 3 (output) = 16,576.
 constexpr int kMlpParams = kMlpHiddenLayers * kMlpIn * kMlpHidden + kMlpHidden * kMlpOut;
-// Packed BF16 image of the weights as the kernels keep them in shared memory:
-// forward operands (4 x 64x64 + 16x64) then backward operands (4 x 64x64 + 64x16).
-constexpr int kMlpPackFwd = kMlpHiddenLayers * 4096 + kMlpOutPad * 64;
-constexpr int kMlpPackElems = 2 * kMlpPackFwd;
+// Packed BF16 image of the weights as the kernels keep them in shared memory
+// (4 x 64x64 + 16x64, the output layer's padding rows zero).
+constexpr int kMlpPackElems = kMlpHiddenLayers * 4096 + kMlpOutPad * 64;
+// The gradient accumulator with the loss behind it.
+constexpr size_t kMlpGradBytes = sizeof(float) * kMlpParams + sizeof(double);
+static_assert(kMlpParams % 2 == 0, "the loss after the gradient must be 8-byte aligned");
 
 struct MlpAdam {
     float lr, beta1, beta2, eps;
@@ -34,7 +37,7 @@ struct MlpState {
     uint16_t *pack;  // kMlpPackElems (BF16 bits)
     float *m, *v;    // kMlpParams
     float *grad;     // kMlpParams
-    double *loss;    // 1
+    double *loss;    // 1, at grad + kMlpParams (one allocation)
     int *err;        // 1
 };
 
