@@ -381,21 +381,16 @@ __global__ void __launch_bounds__(128) k_cw_generate(const __grid_constant__ Dev
 }
 
 template <int L>
-__global__ void __launch_bounds__(128, traverse_blocks(L)) k_cw_extend(const __grid_constant__ DeviceScene s,
-                                                   const __grid_constant__ WfBuffers b, uint32_t cur) {
-    wf::extend<L>(CacheScene{&s}, b, cur);
+__global__ void __launch_bounds__(128, traverse_blocks(L)) k_cw_trace(const __grid_constant__ DeviceScene s,
+                                                                      const __grid_constant__ WfBuffers b,
+                                                                      uint32_t round, float4 *ended) {
+    wf::trace<L>(CacheScene{&s}, b, round, 0, ended);
 }
 
 template <uint32_t C>
 __global__ void __launch_bounds__(128) k_cw_shade(const __grid_constant__ DeviceScene s,
                                                   const __grid_constant__ WfBuffers b, uint32_t cur, float4 *ended) {
     wf::shade<CN, C>(CacheScene{&s}, b, cur, 0, ended);
-}
-
-template <int L>
-__global__ void __launch_bounds__(128, traverse_blocks(L)) k_cw_shadow(const __grid_constant__ DeviceScene s,
-                                                   const __grid_constant__ WfBuffers b, float4 *ended) {
-    wf::shadow<L>(CacheScene{&s}, b, 0, ended);
 }
 
 // Query vertices (the hits of the bounce-`query_depth` rays of queue `cur`).
@@ -509,13 +504,11 @@ cudaError_t launch_cache_frame_wavefront(const DeviceScene &s, const CacheFrameP
                                          uint32_t *suffix_count, cudaStream_t st, unsigned *launches) {
     const uint32_t npix = s.cam.width * s.cam.height;
     if (npix > b.capacity) return cudaErrorInvalidValue;
-    static unsigned g_gen = 0, g_ext = 0, g_shadow = 0, g_query = 0, g_suffix = 0, g_ext2 = 0, g_shadow2 = 0;
+    static unsigned g_gen = 0, g_trace = 0, g_trace2 = 0, g_query = 0, g_suffix = 0;
     if (!g_gen) {
         g_gen = wave_grid(k_cw_generate);
-        g_ext = wave_grid(k_cw_extend<kLevelsFlat>);
-        g_shadow = wave_grid(k_cw_shadow<kLevelsFlat>);
-        g_ext2 = wave_grid(k_cw_extend<kLevelsTwo>);
-        g_shadow2 = wave_grid(k_cw_shadow<kLevelsTwo>);
+        g_trace = wave_grid(k_cw_trace<kLevelsFlat>);
+        g_trace2 = wave_grid(k_cw_trace<kLevelsTwo>);
         g_query = wave_grid(k_cache_query);
         g_suffix = wave_grid(k_cache_suffix);
     }
@@ -524,9 +517,9 @@ cudaError_t launch_cache_frame_wavefront(const DeviceScene &s, const CacheFrameP
     DeviceScene sv = s;
     sv.ip.max_depth = 0xffffffffu;
     const bool two = s.two_level != 0u;
-    auto extend = [&](uint32_t cur) {
-        if (two) k_cw_extend<kLevelsTwo><<<g_ext2, 128, 0, st>>>(sv, b, cur);
-        else k_cw_extend<kLevelsFlat><<<g_ext, 128, 0, st>>>(sv, b, cur);
+    auto trace = [&](uint32_t round) {
+        if (two) k_cw_trace<kLevelsTwo><<<g_trace2, 128, 0, st>>>(sv, b, round, ended);
+        else k_cw_trace<kLevelsFlat><<<g_trace, 128, 0, st>>>(sv, b, round, ended);
     };
     cudaError_t e = cudaMemsetAsync(p.q_rec, 0, sizeof(CacheQueryRec) * npix, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(suffix_count, 0, sizeof(uint32_t), st);
@@ -542,7 +535,7 @@ cudaError_t launch_cache_frame_wavefront(const DeviceScene &s, const CacheFrameP
     ++n;
     for (uint32_t bounce = 0; bounce < p.query_depth; ++bounce) {
         const uint32_t cur = bounce & 1u;
-        extend(cur);
+        trace(bounce);
         cw_shade<0>(mask, sv, b, cur, ended, st, n);
         cw_shade<1>(mask, sv, b, cur, ended, st, n);
         cw_shade<2>(mask, sv, b, cur, ended, st, n);
@@ -550,12 +543,11 @@ cudaError_t launch_cache_frame_wavefront(const DeviceScene &s, const CacheFrameP
         cw_shade<4>(mask, sv, b, cur, ended, st, n);
         cw_shade<5>(mask, sv, b, cur, ended, st, n);
         cw_shade<6>(mask, sv, b, cur, ended, st, n);
-        if (two) k_cw_shadow<kLevelsTwo><<<g_shadow2, 128, 0, st>>>(sv, b, ended);
-        else k_cw_shadow<kLevelsFlat><<<g_shadow, 128, 0, st>>>(sv, b, ended);
-        n += 2;
+        ++n;
     }
+    // The query rays, with the shadow queries of the last bounce.
     const uint32_t cur = p.query_depth & 1u;
-    extend(cur);
+    trace(p.query_depth);
     k_cache_query<<<g_query, 128, 0, st>>>(sv, p, b, cur, ended, suffix_list, suffix_count);
     n += 2;
     if (p.n_train) {

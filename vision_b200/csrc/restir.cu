@@ -1452,14 +1452,10 @@ __global__ void __launch_bounds__(128) k_gi_wf_shade(const __grid_constant__ Dev
     wf::shade<RN, C>(RtScene{&s}, w, cur, 0, radiance);
 }
 
-__global__ void __launch_bounds__(128, kTraverseBlocks) k_gi_wf_extend(const __grid_constant__ DeviceScene s,
-                                                      const __grid_constant__ WfBuffers w, uint32_t cur) {
-    wf::extend<kLevelsFlat>(RtScene{&s}, w, cur);
-}
-
-__global__ void __launch_bounds__(128, kTraverseBlocks) k_gi_wf_shadow(const __grid_constant__ DeviceScene s,
-                                                      const __grid_constant__ WfBuffers w, float4 *radiance) {
-    wf::shadow<kLevelsFlat>(RtScene{&s}, w, 0, radiance);
+__global__ void __launch_bounds__(128, kTraverseBlocks) k_gi_wf_trace(const __grid_constant__ DeviceScene s,
+                                                                      const __grid_constant__ WfBuffers w,
+                                                                      uint32_t round, float4 *radiance) {
+    wf::trace<kLevelsFlat>(RtScene{&s}, w, round, 0, radiance);
 }
 
 // Radiance of each suffix over the BSDF weight, times the chain throughput.
@@ -1777,10 +1773,9 @@ cudaError_t launch_rt_frame(const DeviceScene &s, const RtParams &p, const RtBuf
         n += 3;
     }
     if (wf && radiance) {
-        static unsigned g_ext = 0, g_shadow = 0, g_shade[kWfClasses] = {};
+        static unsigned g_ext = 0, g_shade[kWfClasses] = {};
         if (!g_ext) {
-            g_ext = rt_wave_grid(k_gi_wf_extend);
-            g_shadow = rt_wave_grid(k_gi_wf_shadow);
+            g_ext = rt_wave_grid(k_gi_wf_trace);
             g_shade[0] = rt_wave_grid(k_gi_wf_shade<0>);
             g_shade[1] = rt_wave_grid(k_gi_wf_shade<1>);
             g_shade[2] = rt_wave_grid(k_gi_wf_shade<2>);
@@ -1796,10 +1791,11 @@ cudaError_t launch_rt_frame(const DeviceScene &s, const RtParams &p, const RtBuf
         if (e != cudaSuccess) return e;
         k_gi_wf_start<<<g_pix, 128, 0, st>>>(s, p, b, *wf);
         ++n;
-        for (uint32_t bounce = 0; bounce < p.gi_max_depth; ++bounce) {
+        for (uint32_t bounce = 0; p.gi_max_depth > 0 && bounce <= p.gi_max_depth; ++bounce) {
             const uint32_t cur = bounce & 1u;
-            k_gi_wf_extend<<<g_ext, 128, 0, st>>>(s, *wf, cur);
+            k_gi_wf_trace<<<g_ext, 128, 0, st>>>(s, *wf, bounce, radiance);
             ++n;
+            if (bounce == p.gi_max_depth) break;  // the last bounce's shadow queries
             if (bounce == 0) {
                 k_gi_wf_first<<<g_ext, 128, 0, st>>>(s, b, *wf);
                 ++n;
@@ -1811,8 +1807,6 @@ cudaError_t launch_rt_frame(const DeviceScene &s, const RtParams &p, const RtBuf
             if (mask & 16u) { k_gi_wf_shade<4><<<g_shade[4], 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
             if (mask & 32u) { k_gi_wf_shade<5><<<g_shade[5], 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
             if (mask & 64u) { k_gi_wf_shade<6><<<g_shade[6], 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
-            k_gi_wf_shadow<<<g_shadow, 128, 0, st>>>(s, *wf, radiance);
-            ++n;
         }
         k_gi_wf_finish<<<g_pix, 128, 0, st>>>(s, p, b, radiance);
         ++n;

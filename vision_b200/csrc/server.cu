@@ -8,8 +8,8 @@
 // that arrive while others render start at the next batch and their work
 // overlaps.  A batch is one CUDA-graph launch: the work table upload (pinned
 // host -> device), then the batch's paths as wavefront waves (k_sv_generate
-// maps each slot to its job, scene, pixel and frame; per bounce k_sv_extend,
-// k_sv_shade<C> for every shading class C and k_sv_shadow run the shared
+// maps each slot to its job, scene, pixel and frame; per bounce k_sv_trace and
+// k_sv_shade<C> for every shading class C run the shared
 // wavefront bodies with each slot's own scene), then the film pass
 // k_serve_film (each job's running mean in frame order).  Two graph instances
 // with their own tables, path slots and radiance buffers alternate, so the
@@ -125,11 +125,11 @@ __global__ void __launch_bounds__(128) k_sv_generate(const DeviceScene *scenes, 
     }
 }
 
-__global__ void __launch_bounds__(128) k_sv_extend(const DeviceScene *scenes, const __grid_constant__ WfBuffers b,
-                                                   uint32_t cur) {
+__global__ void __launch_bounds__(128, traverse_blocks(kLevelsAny)) k_sv_trace(const DeviceScene *scenes, const __grid_constant__ WfBuffers b,
+                                                  uint32_t round, uint64_t base, float4 *radiance) {
     __shared__ DeviceScene s_scene[kMaxServeScenes];
     load_scenes(scenes, s_scene);
-    wf::extend<kLevelsAny>(SharedScenes{s_scene}, b, cur);
+    wf::trace<kLevelsAny>(SharedScenes{s_scene}, b, round, base, radiance);
 }
 
 // Shading of class C (0: misses, 1 + MaterialType: hits of that material).
@@ -139,13 +139,6 @@ __global__ void __launch_bounds__(128) k_sv_shade(const DeviceScene *scenes, con
     __shared__ DeviceScene s_scene[kMaxServeScenes];
     load_scenes(scenes, s_scene);
     wf::shade<SN, C>(SharedScenes{s_scene}, b, cur, base, radiance);
-}
-
-__global__ void __launch_bounds__(128) k_sv_shadow(const DeviceScene *scenes, const __grid_constant__ WfBuffers b,
-                                                   uint64_t base, float4 *radiance) {
-    __shared__ DeviceScene s_scene[kMaxServeScenes];
-    load_scenes(scenes, s_scene);
-    wf::shadow<kLevelsAny>(SharedScenes{s_scene}, b, base, radiance);
 }
 
 // NormalRadianceCollector::add_sample (normal.cpp:87-101) per job pixel over
@@ -331,10 +324,10 @@ public:
     cudaError_t capture(uint32_t depth) {
         // One k_sv_shade<C> per shading class, in the graph and here.
         static_assert(kWfClasses == 8, "k_sv_shade launches cover classes 0..7");
-        int sms = 0, per_ext = 0, per_shadow = 0, per_gen = 0, per_shade[kWfClasses] = {};
+        int sms = 0, per_trace = 0, per_gen = 0, per_shade[kWfClasses] = {};
         cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_gen, k_sv_generate, 128, 0);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_ext, k_sv_extend, 128, 0);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_trace, k_sv_trace, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[0], k_sv_shade<0>, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[1], k_sv_shade<1>, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[2], k_sv_shade<2>, 128, 0);
@@ -343,10 +336,9 @@ public:
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[5], k_sv_shade<5>, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[6], k_sv_shade<6>, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[7], k_sv_shade<7>, 128, 0);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shadow, k_sv_shadow, 128, 0);
         if (e != cudaSuccess) return e;
         auto grid_of = [&](int per) { return static_cast<unsigned>(std::max(1, sms * std::max(per, 1))); };
-        const unsigned g_gen = grid_of(per_gen), g_ext = grid_of(per_ext), g_shadow = grid_of(per_shadow);
+        const unsigned g_gen = grid_of(per_gen), g_trace = grid_of(per_trace);
         unsigned g_shade[kWfClasses];
         for (uint32_t c = 0; c < kWfClasses; ++c) g_shade[c] = grid_of(per_shade[c]);
         const unsigned film_grid = static_cast<unsigned>(std::max(1, sms * 4));
@@ -364,9 +356,11 @@ public:
             for (uint64_t w = 0; w < waves; ++w) {
                 const uint64_t base = w * slots;
                 k_sv_generate<<<g_gen, 128, 0, stream>>>(d_scenes, d_tab[k], wfb[k], base, d_rad[k]);
-                for (uint32_t bounce = 0; bounce < depth; ++bounce) {
+                // After the last bounce, its shadow queries.
+                for (uint32_t bounce = 0; bounce <= depth; ++bounce) {
                     const uint32_t cur = bounce & 1u;
-                    k_sv_extend<<<g_ext, 128, 0, stream>>>(d_scenes, wfb[k], cur);
+                    k_sv_trace<<<g_trace, 128, 0, stream>>>(d_scenes, wfb[k], bounce, base, d_rad[k]);
+                    if (bounce == depth) break;
                     k_sv_shade<0><<<g_shade[0], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
                     k_sv_shade<1><<<g_shade[1], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
                     k_sv_shade<2><<<g_shade[2], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
@@ -375,7 +369,6 @@ public:
                     k_sv_shade<5><<<g_shade[5], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
                     k_sv_shade<6><<<g_shade[6], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
                     k_sv_shade<7><<<g_shade[7], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
-                    k_sv_shadow<<<g_shadow, 128, 0, stream>>>(d_scenes, wfb[k], base, d_rad[k]);
                 }
             }
             k_serve_film<<<film_grid, 256, 0, stream>>>(d_tab[k], d_rad[k]);
@@ -385,7 +378,7 @@ public:
         }
         if (e == cudaSuccess) {
             graph_depth = depth;
-            graph_kernels = static_cast<unsigned>(waves * (1 + (2ull + kWfClasses) * depth) + 1);
+            graph_kernels = static_cast<unsigned>(waves * (2 + (1ull + kWfClasses) * depth) + 1);
         }
         return e;
     }

@@ -807,9 +807,10 @@ constexpr int kLevelsFlat = 0, kLevelsTwo = 1, kLevelsAny = 2;
 // 64 registers a thread.  Left alone the compiler takes 96 to 128 of them for
 // the unrolled child test, and with 4 or 5 blocks the passes take 20 % longer
 // (2.1 M camera rays, 2.3 M triangles: 0.50 ms; 8 blocks 0.41, 9 blocks 0.43,
-// 10 blocks 0.47).
+// 10 blocks 0.47).  The two-level kernels call their instance traversals out of
+// line and are asked for 6 (80 registers instead of 146).
 constexpr int kTraverseBlocks = 8;
-constexpr int traverse_blocks(int levels) { return levels == kLevelsFlat ? kTraverseBlocks : 1; }
+constexpr int traverse_blocks(int levels) { return levels == kLevelsFlat ? kTraverseBlocks : 6; }
 
 // One step of the closest-hit traversal; true when the traversal has ended
 // (the result is in t.best_*).

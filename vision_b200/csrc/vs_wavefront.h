@@ -28,9 +28,11 @@ struct WfBuffers {
     float4 *sh_d;    // direction + slot (bits 0..30) and a last-bounce flag (bit 31)
     float4 *sh_c;    // contribution when unoccluded (linear sRGB), w: scene id
     uint32_t *tq;    // hits sorted by shading class: class c at tq[c * capacity]
-    uint32_t *count; // [0], [1]: path queue lengths; [2]: shadow queue length;
-                     // [3 + c]: length of shading class c; [kWfFetchExtend],
-                     // [kWfFetchShadow]: rays handed out by the traversal kernels
+    uint32_t *count; // [cur]: path queue lengths; the rest double-buffered by
+                     // bounce parity k: [kWfShadow + k]: shadow queue length,
+                     // [kWfClass + k * kWfClasses + c]: length of shading class
+                     // c, [kWfFetch + 2 k], [kWfFetch + 2 k + 1]: path and shadow
+                     // rays handed out by the traversal pass
     // Ray binning (all null: off).  Before a traversal pass the queued rays
     // are grouped by a key of direction octant and origin cell: bin_key holds
     // each entry's key, bins 2 x kWfBins counters (sizes, then write
@@ -50,9 +52,10 @@ constexpr uint32_t kWfBins = 1u << kWfBinBits;
 // Shading classes of a hit: 0 = miss, 1 + MaterialType otherwise.  Each class
 // is shaded by its own kernel, compiled with that material's code only.
 constexpr uint32_t kWfClasses = 8;
-constexpr uint32_t kWfFetchExtend = 3 + kWfClasses;
-constexpr uint32_t kWfFetchShadow = kWfFetchExtend + 1;
-constexpr uint32_t kWfCounters = kWfFetchShadow + 1;
+constexpr uint32_t kWfShadow = 2;
+constexpr uint32_t kWfClass = kWfShadow + 2;
+constexpr uint32_t kWfFetch = kWfClass + 2 * kWfClasses;
+constexpr uint32_t kWfCounters = kWfFetch + 4;
 
 // Bytes of device memory per slot of WfBuffers.
 constexpr size_t kWfBytesPerSlot = 6 * 16 + 16 + 16 + 2 * 4 + 3 * 16 + kWfClasses * 4;

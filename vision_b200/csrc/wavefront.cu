@@ -4,11 +4,13 @@
 //   k_wf_generate  camera paths of the wave (PathTracingIntegrator kernel
 //                  body, pt.cpp:53-72): wavelengths, camera ray, queue 0
 //   per bounce:
-//   k_wf_extend    closest hit of every queued ray (traversal only)
+//   k_wf_trace     closest hit of every queued ray, and any hit of the shadow
+//                  queries of the bounce before, with their contribution when
+//                  unoccluded (traversal only; once more after the last
+//                  bounce, for its shadow queries)
 //   k_wf_shade     path_shade: emission, light sample (shadow query), BSDF
 //                  sample, Russian roulette, next ray; survivors to the other
 //                  queue, shadow queries to the shadow queue
-//   k_wf_shadow    any hit of every shadow query, contribution when unoccluded
 //
 // Each slot's sampler draws in the same order as the megakernel (light,
 // BSDF, roulette per bounce) and the radiance is summed in the same order
@@ -43,9 +45,10 @@ __global__ void __launch_bounds__(128) k_wf_generate(const __grid_constant__ Dev
 
 // L: kLevelsFlat or kLevelsTwo, picked on the host from the scene.
 template <int L>
-__global__ void __launch_bounds__(128, traverse_blocks(L)) k_wf_extend(const __grid_constant__ DeviceScene s,
-                                                   const __grid_constant__ WfBuffers b, uint32_t cur) {
-    wf::extend<L>(OneScene{&s}, b, cur);
+__global__ void __launch_bounds__(128, traverse_blocks(L)) k_wf_trace(const __grid_constant__ DeviceScene s,
+                                                                      const __grid_constant__ WfBuffers b,
+                                                                      uint32_t round, uint64_t base, float4 *radiance) {
+    wf::trace<L>(OneScene{&s}, b, round, base, radiance);
 }
 
 // Shading of class C (0: misses, 1 + MaterialType: hits of that material).
@@ -54,13 +57,6 @@ __global__ void __launch_bounds__(128) k_wf_shade(const __grid_constant__ Device
                                                   const __grid_constant__ WfBuffers b, uint32_t cur, uint64_t base,
                                                   float4 *radiance) {
     wf::shade<N, C>(OneScene{&s}, b, cur, base, radiance);
-}
-
-template <int L>
-__global__ void __launch_bounds__(128, traverse_blocks(L)) k_wf_shadow(const __grid_constant__ DeviceScene s,
-                                                   const __grid_constant__ WfBuffers b, uint64_t base,
-                                                   float4 *radiance) {
-    wf::shadow<L>(OneScene{&s}, b, base, radiance);
 }
 
 // ---------------------------------------------------------------------------
@@ -197,20 +193,17 @@ void launch_shade(const ShadeGrids &sg, uint32_t mask, const DeviceScene &s, con
 template <int N>
 cudaError_t wave_loop(const DeviceScene &s, uint32_t frame_begin, uint64_t paths, float4 *radiance,
                       const WfBuffers &b, uint32_t class_mask, cudaStream_t st, unsigned *launches) {
-    static std::atomic<int> g_gen[64], g_ext[64], g_shadow[64], g_ext2[64], g_shadow2[64];
+    static std::atomic<int> g_gen[64], g_trace[64], g_trace2[64];
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    unsigned grid_gen, grid_ext, grid_shadow;
+    unsigned grid_gen, grid_trace;
     ShadeGrids sg{};
     if ((e = resident_grid(k_wf_generate<N>, dev, g_gen[dev], &grid_gen)) != cudaSuccess) return e;
     const bool two = s.two_level != 0u;
-    if ((e = two ? resident_grid(k_wf_extend<kLevelsTwo>, dev, g_ext2[dev], &grid_ext)
-                 : resident_grid(k_wf_extend<kLevelsFlat>, dev, g_ext[dev], &grid_ext)) != cudaSuccess)
-        return e;
-    if ((e = two ? resident_grid(k_wf_shadow<kLevelsTwo>, dev, g_shadow2[dev], &grid_shadow)
-                 : resident_grid(k_wf_shadow<kLevelsFlat>, dev, g_shadow[dev], &grid_shadow)) != cudaSuccess)
+    if ((e = two ? resident_grid(k_wf_trace<kLevelsTwo>, dev, g_trace2[dev], &grid_trace)
+                 : resident_grid(k_wf_trace<kLevelsFlat>, dev, g_trace[dev], &grid_trace)) != cudaSuccess)
         return e;
     if ((e = shade_grid<N, 0>(dev, sg)) != cudaSuccess) return e;
     if ((e = shade_grid<N, 1>(dev, sg)) != cudaSuccess) return e;
@@ -227,30 +220,34 @@ cudaError_t wave_loop(const DeviceScene &s, uint32_t frame_begin, uint64_t paths
     int sms = 0;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     const unsigned grid_bin = static_cast<unsigned>(sms) * 8u;
-    // The traversal passes read the binned queue (path slots) or the shadow
-    // permutation instead of the queues in push order.
-    WfBuffers bs = b;
-    bs.sh_perm = binning ? b.sh_perm : nullptr;
     for (uint64_t base = 0; base < paths; base += b.capacity) {
         const uint32_t n = static_cast<uint32_t>(std::min<uint64_t>(b.capacity, paths - base));
         const unsigned g = std::min<unsigned>(grid_gen, (n + 127u) / 128u);
         k_wf_generate<N><<<g, 128, 0, st>>>(s, b, frame_begin, base, n, radiance);
         ++n_launch;
-        for (uint32_t bounce = 0; bounce < s.ip.max_depth; ++bounce) {
-            const uint32_t cur = bounce & 1u;
-            // Camera rays (bounce 0) arrive in pixel order, already coherent.
-            const bool bin_paths = binning && bounce > 0;
-            WfBuffers be = b;
-            be.sh_perm = nullptr;
-            if (bin_paths) {
+        for (uint32_t round = 0; s.ip.max_depth > 0 && round <= s.ip.max_depth; ++round) {
+            const uint32_t cur = round & 1u;
+            // The traversal pass reads the binned queue (path slots) and the
+            // shadow permutation instead of the queues in push order.  Camera
+            // rays (round 0) arrive in pixel order, already coherent.
+            WfBuffers bt = b;
+            bt.sh_perm = nullptr;
+            if (binning && round > 0) {
+                const uint32_t *shadows = b.count + kWfShadow + (cur ^ 1u);
                 k_bin_count<<<grid_bin, 256, 0, st>>>(s, b.count + cur, b.queue[cur], b.o, b.d, b.bin_key, b.bins);
                 k_bin_scan<<<1, 1024, 0, st>>>(b.bins);
                 k_bin_scatter<<<grid_bin, 256, 0, st>>>(b.count + cur, b.queue[cur], b.bin_key, b.bins, b.binned);
-                be.queue[cur] = b.binned;
-                n_launch += 3;
+                k_bin_count<<<grid_bin, 256, 0, st>>>(s, shadows, nullptr, b.sh_o, b.sh_d, b.bin_key, b.bins);
+                k_bin_scan<<<1, 1024, 0, st>>>(b.bins);
+                k_bin_scatter<<<grid_bin, 256, 0, st>>>(shadows, nullptr, b.bin_key, b.bins, b.sh_perm);
+                bt.queue[cur] = b.binned;
+                bt.sh_perm = b.sh_perm;
+                n_launch += 6;
             }
-            if (two) k_wf_extend<kLevelsTwo><<<grid_ext, 128, 0, st>>>(s, be, cur);
-            else k_wf_extend<kLevelsFlat><<<grid_ext, 128, 0, st>>>(s, be, cur);
+            if (two) k_wf_trace<kLevelsTwo><<<grid_trace, 128, 0, st>>>(s, bt, round, base, radiance);
+            else k_wf_trace<kLevelsFlat><<<grid_trace, 128, 0, st>>>(s, bt, round, base, radiance);
+            ++n_launch;
+            if (round == s.ip.max_depth) break;
             launch_shade<N, 0>(sg, mask, s, b, cur, base, radiance, st, n_launch);
             launch_shade<N, 1>(sg, mask, s, b, cur, base, radiance, st, n_launch);
             launch_shade<N, 2>(sg, mask, s, b, cur, base, radiance, st, n_launch);
@@ -259,15 +256,6 @@ cudaError_t wave_loop(const DeviceScene &s, uint32_t frame_begin, uint64_t paths
             launch_shade<N, 5>(sg, mask, s, b, cur, base, radiance, st, n_launch);
             launch_shade<N, 6>(sg, mask, s, b, cur, base, radiance, st, n_launch);
             launch_shade<N, 7>(sg, mask, s, b, cur, base, radiance, st, n_launch);
-            if (binning) {
-                k_bin_count<<<grid_bin, 256, 0, st>>>(s, b.count + 2, nullptr, b.sh_o, b.sh_d, b.bin_key, b.bins);
-                k_bin_scan<<<1, 1024, 0, st>>>(b.bins);
-                k_bin_scatter<<<grid_bin, 256, 0, st>>>(b.count + 2, nullptr, b.bin_key, b.bins, b.sh_perm);
-                n_launch += 3;
-            }
-            if (two) k_wf_shadow<kLevelsTwo><<<grid_shadow, 128, 0, st>>>(s, bs, base, radiance);
-            else k_wf_shadow<kLevelsFlat><<<grid_shadow, 128, 0, st>>>(s, bs, base, radiance);
-            n_launch += 2;
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
