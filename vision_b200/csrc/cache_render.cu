@@ -538,7 +538,6 @@ cudaError_t launch_cache_frame_wavefront(const DeviceScene &s, const CacheFrameP
         trace(bounce);
         cw_shade<0>(mask, sv, b, cur, ended, st, n);
         cw_shade<1>(mask, sv, b, cur, ended, st, n);
-        cw_shade<2>(mask, sv, b, cur, ended, st, n);
         cw_shade<3>(mask, sv, b, cur, ended, st, n);
         cw_shade<4>(mask, sv, b, cur, ended, st, n);
         cw_shade<5>(mask, sv, b, cur, ended, st, n);

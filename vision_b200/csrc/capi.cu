@@ -414,7 +414,8 @@ bool has_mix(const HostScene &h) {
 
 uint32_t shading_classes(const HostScene &h) {
     uint32_t m = 1u;
-    for (const Material &mt : h.materials) m |= 1u << (1u + mt.type);
+    for (const Material &mt : h.materials)
+        if (mt.type != kMatBlackBody) m |= 1u << (1u + mt.type);  // emitters end paths in class 0
     return m;
 }
 
@@ -1259,7 +1260,7 @@ int restir_frame_locked(vs_scene *s, uint32_t frame_index, uint32_t film_index, 
     // Scenes of diffuse surfaces and emitters only take the kernels compiled
     // for those materials alone.
     const uint32_t classes = shading_classes(s->host);
-    const uint32_t diffuse_only = 1u | (1u << (1u + kMatDiffuse)) | (1u << (1u + kMatBlackBody));
+    const uint32_t diffuse_only = 1u | (1u << (1u + kMatDiffuse));
     auto launch = (classes & ~diffuse_only) == 0u ? rt_diffuse::launch_rt_frame : rt_all::launch_rt_frame;
     VS_CUDA(launch(s->device_view(), p, s->rt.view(), film_index, s->film32.ptr, wavefront ? &wfv : nullptr,
                    wavefront ? s->radiance.ptr : nullptr, classes, st, &n),

@@ -1778,7 +1778,6 @@ cudaError_t launch_rt_frame(const DeviceScene &s, const RtParams &p, const RtBuf
             g_ext = rt_wave_grid(k_gi_wf_trace);
             g_shade[0] = rt_wave_grid(k_gi_wf_shade<0>);
             g_shade[1] = rt_wave_grid(k_gi_wf_shade<1>);
-            g_shade[2] = rt_wave_grid(k_gi_wf_shade<2>);
             g_shade[3] = rt_wave_grid(k_gi_wf_shade<3>);
             g_shade[4] = rt_wave_grid(k_gi_wf_shade<4>);
             g_shade[5] = rt_wave_grid(k_gi_wf_shade<5>);
@@ -1802,7 +1801,6 @@ cudaError_t launch_rt_frame(const DeviceScene &s, const RtParams &p, const RtBuf
             }
             if (mask & 1u) { k_gi_wf_shade<0><<<g_shade[0], 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
             if (mask & 2u) { k_gi_wf_shade<1><<<g_shade[1], 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
-            if (mask & 4u) { k_gi_wf_shade<2><<<g_shade[2], 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
             if (mask & 8u) { k_gi_wf_shade<3><<<g_shade[3], 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
             if (mask & 16u) { k_gi_wf_shade<4><<<g_shade[4], 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
             if (mask & 32u) { k_gi_wf_shade<5><<<g_shade[5], 128, 0, st>>>(s, *wf, cur, radiance); ++n; }

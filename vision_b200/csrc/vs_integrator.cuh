@@ -357,7 +357,10 @@ struct ShadowQuery {
 // (the megakernel: nothing of the query stays live across the BSDF code), and
 // add its contribution to ps.L; sq then stays invalid.  M: the material types
 // compiled in (kAllMaterials, or one class for the material-sorted wavefront
-// kernels, whose hits all have that type); M = 0 compiles the miss only.
+// kernels, whose hits all have that type).  A non-scattering emitter's lobe
+// (BlackBodyLobe) is zero, so a path adds its emission and ends there: its
+// light sample would add nothing and its throughput becomes zero.  M = that
+// material only compiles just this and the miss.
 //
 // path_shade_acc generalises the gathering: every contribution (spectral,
 // already weighted) goes through acc(ps, c) — RgbAcc adds its linear sRGB to
@@ -415,13 +418,14 @@ __device__ __forceinline__ bool path_shade_acc(const DeviceScene &s, PathState<N
     const IntegratorParams &ip = s.ip;
     const uint32_t bounce = ps.bounce;
     sq.valid = false;
-    if (!hit_any || M == 0u) {
+    if (!hit_any) {
         miss_emission<N>(s, ps, acc);
         return false;
     }
     Interaction it = surface_interaction(s, hit, ps.rd, true);
     if (first && bounce == 0) *first = it;
     if (emit) hit_emission<N>(s, ps, it, acc);
+    if constexpr (M == 1u << kMatBlackBody) return false;
     // Light sample: 1 draw for the light, 2 for the surface point.
     float u_light = ps.smp.next();
     f2 u_surf = ps.smp.next2();

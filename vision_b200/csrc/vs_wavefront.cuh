@@ -195,7 +195,11 @@ __device__ __forceinline__ void trace(const Scenes &scenes, const WfBuffers &b, 
             if (!__any_sync(0xffffffffu, active)) break;
             if (active && closest_step<Levels>(*s, r, t, stack)) {
                 const Hit h = trav_hit(*s, t);
-                const uint32_t cls = h.inst_id == kInvalid ? 0u : 1u + s->materials[s->instances[h.inst_id].mat_id].type;
+                uint32_t cls = 0u;
+                if (h.inst_id != kInvalid) {
+                    const uint32_t type = s->materials[s->instances[h.inst_id].mat_id].type;
+                    if (type != kMatBlackBody) cls = 1u + type;
+                }
                 b.hit[slot] = h;
                 b.tq[static_cast<size_t>(cls) * b.capacity + class_push(b.count + kWfClass + cur * kWfClasses, cls)] =
                     slot;
@@ -248,7 +252,7 @@ __device__ __forceinline__ void trace(const Scenes &scenes, const WfBuffers &b, 
 // The shading-class mask of path_shade for class C.
 template <uint32_t C>
 struct ClassMask {
-    static constexpr uint32_t value = C == 0u ? 0u : (1u << (C - 1u));
+    static constexpr uint32_t value = C == 0u ? 1u << kMatBlackBody : 1u << (C - 1u);
 };
 
 // One bounce (path_shade) of every path of shading class C after its closest
@@ -267,7 +271,8 @@ __device__ __forceinline__ void shade(const Scenes &scenes, const WfBuffers &b, 
         const DeviceScene &s = scenes(scene);
         const Hit h = b.hit[slot];
         ShadowQuery sq;
-        bool more = path_shade<N, false, ClassMask<C>::value>(s, ps, C != 0u, h, nullptr, sq);
+        bool more =
+            path_shade<N, false, ClassMask<C>::value>(s, ps, C != 0u || h.inst_id != kInvalid, h, nullptr, sq);
         if (more) more = ++ps.bounce < s.ip.max_depth;
         if (more) {
             store<N>(b, slot, ps, scene);

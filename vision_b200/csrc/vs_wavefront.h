@@ -49,8 +49,10 @@ struct WfBuffers {
 constexpr uint32_t kWfBinBits = 12;
 constexpr uint32_t kWfBins = 1u << kWfBinBits;
 
-// Shading classes of a hit: 0 = miss, 1 + MaterialType otherwise.  Each class
-// is shaded by its own kernel, compiled with that material's code only.
+// Shading classes of a hit: 0 = the path ends here (a miss, or an emitter
+// surface that does not scatter), 1 + MaterialType otherwise (so class 1 +
+// kMatBlackBody stays empty and has no kernel).  Each class is shaded by its
+// own kernel, compiled with that material's code only.
 constexpr uint32_t kWfClasses = 8;
 constexpr uint32_t kWfShadow = 2;
 constexpr uint32_t kWfClass = kWfShadow + 2;
@@ -63,8 +65,8 @@ constexpr size_t kWfBytesPerSlot = 6 * 16 + 16 + 16 + 2 * 4 + 3 * 16 + kWfClasse
 // Renders the paths of frames [frame_begin, frame_begin + frame_count) into
 // radiance[] (one float4 per path, frame-major, as launch_render) in waves of
 // at most b.capacity paths.  `launches` gets the number of kernels launched.
-// class_mask: bit c set when shading class c can occur (bit 0, misses, is
-// always launched); classes without a bit are not launched.
+// class_mask: bit c set when shading class c can occur (bit 0, ended paths,
+// is always launched); classes without a bit are not launched.
 cudaError_t launch_render_wavefront(const DeviceScene &s, uint32_t frame_begin, uint32_t frame_count,
                                     float4 *radiance, const WfBuffers &b, uint32_t class_mask, cudaStream_t st,
                                     unsigned *launches);

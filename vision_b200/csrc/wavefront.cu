@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(128, traverse_blocks(L)) k_wf_trace(const __gr
     wf::trace<L>(OneScene{&s}, b, round, base, radiance);
 }
 
-// Shading of class C (0: misses, 1 + MaterialType: hits of that material).
+// Shading of class C (0: paths that end, 1 + MaterialType: hits of that material).
 template <int N, uint32_t C>
 __global__ void __launch_bounds__(128) k_wf_shade(const __grid_constant__ DeviceScene s,
                                                   const __grid_constant__ WfBuffers b, uint32_t cur, uint64_t base,
@@ -207,7 +207,6 @@ cudaError_t wave_loop(const DeviceScene &s, uint32_t frame_begin, uint64_t paths
         return e;
     if ((e = shade_grid<N, 0>(dev, sg)) != cudaSuccess) return e;
     if ((e = shade_grid<N, 1>(dev, sg)) != cudaSuccess) return e;
-    if ((e = shade_grid<N, 2>(dev, sg)) != cudaSuccess) return e;
     if ((e = shade_grid<N, 3>(dev, sg)) != cudaSuccess) return e;
     if ((e = shade_grid<N, 4>(dev, sg)) != cudaSuccess) return e;
     if ((e = shade_grid<N, 5>(dev, sg)) != cudaSuccess) return e;
@@ -250,7 +249,6 @@ cudaError_t wave_loop(const DeviceScene &s, uint32_t frame_begin, uint64_t paths
             if (round == s.ip.max_depth) break;
             launch_shade<N, 0>(sg, mask, s, b, cur, base, radiance, st, n_launch);
             launch_shade<N, 1>(sg, mask, s, b, cur, base, radiance, st, n_launch);
-            launch_shade<N, 2>(sg, mask, s, b, cur, base, radiance, st, n_launch);
             launch_shade<N, 3>(sg, mask, s, b, cur, base, radiance, st, n_launch);
             launch_shade<N, 4>(sg, mask, s, b, cur, base, radiance, st, n_launch);
             launch_shade<N, 5>(sg, mask, s, b, cur, base, radiance, st, n_launch);
