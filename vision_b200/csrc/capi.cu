@@ -1468,6 +1468,7 @@ int vs_server_add_scene(vs_server *s, vs_scene *scene, uint32_t *scene_id) {
     if (!s || !scene || !scene_id) return VS_E_INVALID;
     DeviceScene dv;
     uint64_t bytes = 0;
+    uint32_t classes = 0;
     bool rt = false;
     Camera cam{};
     const float4 *film = nullptr;
@@ -1487,6 +1488,7 @@ int vs_server_add_scene(vs_server *s, vs_scene *scene, uint32_t *scene_id) {
         } else {
             dv = scene->device_view();
             bytes = scene->device_bytes();
+            classes = shading_classes(scene->host);
         }
     }
     std::string err;
@@ -1507,7 +1509,7 @@ int vs_server_add_scene(vs_server *s, vs_scene *scene, uint32_t *scene_id) {
         };
         rc = server_add_rt_scene(s->impl, cam, bytes, std::move(hooks), scene_id, err);
     } else {
-        rc = server_add_scene(s->impl, dv, bytes, scene_id, err);
+        rc = server_add_scene(s->impl, dv, classes, bytes, scene_id, err);
     }
     return rc == VS_OK ? VS_OK : s->fail(rc, err);
 }

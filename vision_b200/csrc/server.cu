@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(128, traverse_blocks(kLevelsAny)) k_sv_trace(c
     wf::trace<kLevelsAny>(SharedScenes{s_scene}, b, round, base, radiance);
 }
 
-// Shading of class C (0: misses, 1 + MaterialType: hits of that material).
+// Shading of class C (0: paths that end, 1 + MaterialType: hits of that material).
 template <uint32_t C>
 __global__ void __launch_bounds__(128) k_sv_shade(const DeviceScene *scenes, const __grid_constant__ WfBuffers b,
                                                   uint32_t cur, uint64_t base, float4 *radiance) {
@@ -214,6 +214,8 @@ public:
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     uint32_t graph_depth = 0;   // bounce iterations captured in the graphs
     uint32_t need_depth = 0;    // largest max_depth of the resident scenes
+    uint32_t graph_classes = 0; // shading classes captured in the graphs
+    uint32_t need_classes = 1u; // shading classes of the resident scenes (0 always)
     unsigned graph_kernels = 0; // kernel nodes per graph
     cudaEvent_t ev_start[2] = {nullptr, nullptr}, ev_end[2] = {nullptr, nullptr};
 
@@ -277,7 +279,7 @@ public:
             if (e == cudaSuccess) e = cudaEventCreate(&ev_end[k]);
         }
         for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = alloc_slots(k);
-        if (e == cudaSuccess) e = capture(1);
+        if (e == cudaSuccess) e = capture(1, need_classes);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e == cudaSuccess) worker = std::thread([this] { run(); });
         return e;
@@ -319,18 +321,17 @@ public:
         return cudaSuccess;
     }
 
-    // (Re)captures both batch graphs with `depth` bounce iterations per wave.
-    // No batch may be in flight.
-    cudaError_t capture(uint32_t depth) {
-        // One k_sv_shade<C> per shading class, in the graph and here.
-        static_assert(kWfClasses == 8, "k_sv_shade launches cover classes 0..7");
+    // (Re)captures both batch graphs with `depth` bounce iterations per wave
+    // and the shading passes of `classes`.  No batch may be in flight.
+    cudaError_t capture(uint32_t depth, uint32_t classes) {
+        // One k_sv_shade<C> per shading class that has a kernel, in the graph and here.
+        static_assert(kWfClasses == 8 && kMatBlackBody == 1, "k_sv_shade launches cover classes 0, 1 and 3..7");
         int sms = 0, per_trace = 0, per_gen = 0, per_shade[kWfClasses] = {};
         cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_gen, k_sv_generate, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_trace, k_sv_trace, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[0], k_sv_shade<0>, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[1], k_sv_shade<1>, 128, 0);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[2], k_sv_shade<2>, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[3], k_sv_shade<3>, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[4], k_sv_shade<4>, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[5], k_sv_shade<5>, 128, 0);
@@ -361,14 +362,13 @@ public:
                     const uint32_t cur = bounce & 1u;
                     k_sv_trace<<<g_trace, 128, 0, stream>>>(d_scenes, wfb[k], bounce, base, d_rad[k]);
                     if (bounce == depth) break;
-                    k_sv_shade<0><<<g_shade[0], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
-                    k_sv_shade<1><<<g_shade[1], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
-                    k_sv_shade<2><<<g_shade[2], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
-                    k_sv_shade<3><<<g_shade[3], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
-                    k_sv_shade<4><<<g_shade[4], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
-                    k_sv_shade<5><<<g_shade[5], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
-                    k_sv_shade<6><<<g_shade[6], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
-                    k_sv_shade<7><<<g_shade[7], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
+                    if ((classes >> 0) & 1u) k_sv_shade<0><<<g_shade[0], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
+                    if ((classes >> 1) & 1u) k_sv_shade<1><<<g_shade[1], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
+                    if ((classes >> 3) & 1u) k_sv_shade<3><<<g_shade[3], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
+                    if ((classes >> 4) & 1u) k_sv_shade<4><<<g_shade[4], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
+                    if ((classes >> 5) & 1u) k_sv_shade<5><<<g_shade[5], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
+                    if ((classes >> 6) & 1u) k_sv_shade<6><<<g_shade[6], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
+                    if ((classes >> 7) & 1u) k_sv_shade<7><<<g_shade[7], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
                 }
             }
             k_serve_film<<<film_grid, 256, 0, stream>>>(d_tab[k], d_rad[k]);
@@ -378,7 +378,10 @@ public:
         }
         if (e == cudaSuccess) {
             graph_depth = depth;
-            graph_kernels = static_cast<unsigned>(waves * (2 + (1ull + kWfClasses) * depth) + 1);
+            graph_classes = classes;
+            uint64_t passes = 0;
+            for (uint32_t c = 0; c < kWfClasses; ++c) passes += (classes >> c) & 1u;
+            graph_kernels = static_cast<unsigned>(waves * (2 + (1ull + passes) * depth) + 1);
         }
         return e;
     }
@@ -472,14 +475,15 @@ public:
                 continue;
             }
             if (inflight.size() >= 2) complete_oldest();
-            uint32_t depth;
+            uint32_t depth, classes;
             {
                 std::lock_guard<std::mutex> lk(mu);
                 depth = need_depth;
+                classes = need_classes;
             }
-            if (depth > graph_depth) {
+            if (depth > graph_depth || (classes & ~graph_classes) != 0u) {
                 while (!inflight.empty()) complete_oldest();
-                cudaError_t e = capture(depth);
+                cudaError_t e = capture(std::max(depth, graph_depth), classes);
                 if (e != cudaSuccess) {
                     std::lock_guard<std::mutex> lk(mu);
                     fail_locked(std::string("server graph capture: ") + cudaGetErrorString(e));
@@ -623,7 +627,8 @@ int server_create(int device, uint64_t hbm_budget, uint32_t max_jobs, uint64_t p
 
 void server_destroy(Server *s) { delete s; }
 
-int server_add_scene(Server *s, const DeviceScene &scene, uint64_t bytes, uint32_t *id, std::string &err) {
+int server_add_scene(Server *s, const DeviceScene &scene, uint32_t classes, uint64_t bytes, uint32_t *id,
+                     std::string &err) {
     std::lock_guard<std::mutex> lk(s->mu);
     if (s->nscenes >= kMaxServeScenes) {
         err = "too many resident scenes";
@@ -647,6 +652,7 @@ int server_add_scene(Server *s, const DeviceScene &scene, uint64_t bytes, uint32
     }
     s->scene_cam[s->nscenes] = scene.cam;
     s->need_depth = std::max(s->need_depth, scene.ip.max_depth);
+    s->need_classes |= classes;
     s->resident += bytes;
     s->st.resident_bytes = s->resident;
     *id = s->nscenes++;

@@ -55,9 +55,10 @@ class Server;
 int server_create(int device, uint64_t hbm_budget, uint32_t max_jobs, uint64_t paths_per_batch, Server **out,
                   std::string &err);
 void server_destroy(Server *s);
-// `bytes`: the scene's device memory, counted against the HBM budget for as
+// `classes`: its shading classes (bit c set when class c can occur), the only
+// ones the batches then launch.  `bytes`: the scene's device memory, counted against the HBM budget for as
 // long as the server holds the scene.
-int server_add_scene(Server *s, const DeviceScene &scene, uint64_t bytes, uint32_t *id, std::string &err);
+int server_add_scene(Server *s, const DeviceScene &scene, uint32_t classes, uint64_t bytes, uint32_t *id, std::string &err);
 // A real-time scene: `bytes` counts its geometry and its resident per-pixel
 // buffers (reservoirs, surfaces, film), all allocated before the call.  Jobs
 // on it render at the scene's resolution, one frame per batch, in submission
