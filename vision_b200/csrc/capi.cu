@@ -419,6 +419,24 @@ uint32_t shading_classes(const HostScene &h) {
     return m;
 }
 
+// Whether vs_render's wavefront schedule renders `paths` paths with the
+// persistent megakernel instead (the same films, bit for bit).  A wavefront
+// bounce is a traversal pass and one shading pass per class, each of which
+// lasts as long as its slowest warp however few paths it has; the megakernel
+// has no such steps but runs all materials' code at low occupancy.  Measured
+// crossing points (us, wavefront / megakernel): box room of depth 8, diffuse,
+// 519 / 397 at 65,536 paths and 572 / 676 at 131,044; rooms with principled
+// or glass and metal, depth 8, 739 / 378 and 1053 / 464 at 4,096 paths,
+// 768 / 882 and 1078 / 1081 at 16,384; the large scene, depth 16, 3145 / 1485
+// at 16,384, 3705 / 3049 at 65,536 and 4473 / 8245 at 262,144.  The wavefront's
+// cost grows with the depth until roulette has ended most paths.  (Mix
+// materials render in wavefront form only.)
+bool small_render(const HostScene &h, uint64_t paths) {
+    if (has_mix(h)) return false;
+    const bool diffuse = (shading_classes(h) & ~(1u | (1u << (1u + kMatDiffuse)))) == 0u;
+    return paths <= std::min<uint64_t>(h.ip.max_depth, 16u) * (diffuse ? 8192u : 1536u);
+}
+
 // Per instance: the world-to-object rows and (mesh root node, first
 // primitive) as bits (DeviceScene::inst_xf).
 std::vector<float4> instance_transforms(const HostScene &h) {
@@ -811,8 +829,11 @@ int vs_render(vs_scene *s, uint32_t frame_begin, uint32_t frame_count, int film_
     if (frames_per_chunk == 0) return fail(ctx, VS_E_RANGE, "resolution above the per-launch path limit");
     if (frames_per_chunk > frame_count) frames_per_chunk = frame_count;
     VS_CUDA(s->radiance.alloc(static_cast<size_t>(frames_per_chunk * npix)), "radiance alloc");
-    if (s->schedule == VS_SCHEDULE_PERSISTENT) VS_CUDA(s->path_counter.alloc(1), "path counter alloc");
-    const bool wavefront = s->schedule == VS_SCHEDULE_WAVEFRONT || s->schedule == VS_SCHEDULE_WAVEFRONT_BINNED;
+    const bool small = s->schedule == VS_SCHEDULE_WAVEFRONT && small_render(s->host, frames_per_chunk * npix);
+    const bool persistent = s->schedule == VS_SCHEDULE_PERSISTENT || small;
+    if (persistent) VS_CUDA(s->path_counter.alloc(1), "path counter alloc");
+    const bool wavefront =
+        !small && (s->schedule == VS_SCHEDULE_WAVEFRONT || s->schedule == VS_SCHEDULE_WAVEFRONT_BINNED);
     if (!wavefront && has_mix(s->host))
         return fail(ctx, VS_E_UNSUPPORTED, "mix / add materials render with the wavefront schedules only");
     if (wavefront)
@@ -840,7 +861,7 @@ int vs_render(vs_scene *s, uint32_t frame_begin, uint32_t frame_count, int film_
             add_launches(n);
         } else {
             VS_CUDA(launch_render(dv, frame_begin + f, fc, s->radiance.ptr, st,
-                                  s->schedule == VS_SCHEDULE_PERSISTENT ? s->path_counter.ptr : nullptr),
+                                  persistent ? s->path_counter.ptr : nullptr),
                     "render launch");
         }
         if (s->timing) VS_CUDA(timed_event(s->ev_render), "timing event");
