@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "vs_host.h"
+#include "vs_host_copy.h"
 #include "vs_launch.h"
 #include "vs_microfacet.h"
 #include "vs_cache_render.h"
@@ -24,6 +25,7 @@ struct vs_context {
     mutable std::mutex mu;
     std::string error;
     bool consts_uploaded = false;
+    HostCopy download;  // films and frame buffers to host memory
 };
 
 namespace {
@@ -922,26 +924,25 @@ int vs_film_download(vs_scene *s, void *dst, size_t bytes, int which) {
                     "picture");
             src = s->exposed.ptr;
         }
-        VS_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st), "film copy");
+        VS_CUDA(ctx->download.copy(dst, src, bytes, ctx->device, st), "film copy");
     } else if (which == VS_FILM_RGBA8) {
         if (bytes != npix * 4) return fail(ctx, VS_E_INVALID, "film size mismatch");
         uchar4 *out8 = reinterpret_cast<uchar4 *>(s->exposed.ptr);
         VS_CUDA(launch_picture(s->film32.ptr, static_cast<uint32_t>(npix), s->host.cam.exposure, s->host.tone_mapper, 2u,
                                true, nullptr, out8, st),
                 "picture");
-        VS_CUDA(cudaMemcpyAsync(dst, out8, bytes, cudaMemcpyDeviceToHost, st), "film copy");
+        VS_CUDA(ctx->download.copy(dst, out8, bytes, ctx->device, st), "film copy");
     } else if (which == VS_FILM_SUM64) {
         if (!s->film64_valid) return fail(ctx, VS_E_STATE, "FP64 film not rendered");
         if (bytes != npix * 32) return fail(ctx, VS_E_INVALID, "film size mismatch");
-        VS_CUDA(cudaMemcpyAsync(dst, s->film64.ptr, bytes, cudaMemcpyDeviceToHost, st), "film copy");
+        VS_CUDA(ctx->download.copy(dst, s->film64.ptr, bytes, ctx->device, st), "film copy");
     } else if (which == VS_FILM_SUMSQ64) {
         if (!s->film64sq_valid) return fail(ctx, VS_E_STATE, "FP64 film with squares not rendered (vs_render, FP64)");
         if (bytes != npix * 32) return fail(ctx, VS_E_INVALID, "film size mismatch");
-        VS_CUDA(cudaMemcpyAsync(dst, s->film64.ptr + npix * 4, bytes, cudaMemcpyDeviceToHost, st), "film copy");
+        VS_CUDA(ctx->download.copy(dst, s->film64.ptr + npix * 4, bytes, ctx->device, st), "film copy");
     } else {
         return fail(ctx, VS_E_INVALID, "unknown film buffer");
     }
-    VS_CUDA(cudaStreamSynchronize(st), "film sync");
     return VS_OK;
 }
 
@@ -1425,8 +1426,7 @@ int vs_restir_download(vs_scene *s, int which, void *dst, size_t bytes) {
     }
     if (bytes != n * elem) return fail(ctx, VS_E_INVALID, "ReSTIR buffer size mismatch");
     VS_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
-    VS_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream), "restir copy");
-    VS_CUDA(cudaStreamSynchronize(ctx->stream), "restir sync");
+    VS_CUDA(ctx->download.copy(dst, src, bytes, ctx->device, ctx->stream), "restir copy");
     return VS_OK;
 }
 
@@ -1905,8 +1905,7 @@ int vs_cache_download(vs_scene *s, int which, void *dst, size_t bytes) {
     if (bytes != n * elem) return fail(ctx, VS_E_INVALID, "cache buffer size mismatch");
     if (n == 0) return VS_OK;
     VS_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
-    VS_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream), "cache copy");
-    VS_CUDA(cudaStreamSynchronize(ctx->stream), "cache sync");
+    VS_CUDA(ctx->download.copy(dst, src, bytes, ctx->device, ctx->stream), "cache copy");
     return VS_OK;
 }
 
