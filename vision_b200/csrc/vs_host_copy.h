@@ -10,7 +10,7 @@ namespace vs {
 // (a new film array's pages are faulted and zeroed by that write) at 10 to 15
 // GB/s, a quarter of what the bus delivers.  Here the device writes chunks
 // into a page-locked ring and several threads take them in order from there.
-// The ring (8 MB) and the threads are made by the first copy that uses them
+// The ring (4 MB) and the threads are made by the first copy that uses them
 // and live as long as the object; copies of one object run one at a time.
 class HostCopy {
 public:
