@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(128, traverse_blocks(kLevelsAny)) k_sv_trace(c
 
 // Shading of class C (0: paths that end, 1 + MaterialType: hits of that material).
 template <uint32_t C>
-__global__ void __launch_bounds__(128) k_sv_shade(const DeviceScene *scenes, const __grid_constant__ WfBuffers b,
+__global__ void __launch_bounds__(shade_threads(C)) k_sv_shade(const DeviceScene *scenes, const __grid_constant__ WfBuffers b,
                                                   uint32_t cur, uint64_t base, float4 *radiance) {
     __shared__ DeviceScene s_scene[kMaxServeScenes];
     load_scenes(scenes, s_scene);
@@ -334,7 +334,7 @@ public:
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[1], k_sv_shade<1>, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[3], k_sv_shade<3>, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[4], k_sv_shade<4>, 128, 0);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[5], k_sv_shade<5>, 128, 0);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[5], k_sv_shade<5>, shade_threads(5), 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[6], k_sv_shade<6>, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_shade[7], k_sv_shade<7>, 128, 0);
         if (e != cudaSuccess) return e;
@@ -366,7 +366,7 @@ public:
                     if ((classes >> 1) & 1u) k_sv_shade<1><<<g_shade[1], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
                     if ((classes >> 3) & 1u) k_sv_shade<3><<<g_shade[3], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
                     if ((classes >> 4) & 1u) k_sv_shade<4><<<g_shade[4], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
-                    if ((classes >> 5) & 1u) k_sv_shade<5><<<g_shade[5], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
+                    if ((classes >> 5) & 1u) k_sv_shade<5><<<g_shade[5], shade_threads(5), 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
                     if ((classes >> 6) & 1u) k_sv_shade<6><<<g_shade[6], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
                     if ((classes >> 7) & 1u) k_sv_shade<7><<<g_shade[7], 128, 0, stream>>>(d_scenes, wfb[k], cur, base, d_rad[k]);
                 }

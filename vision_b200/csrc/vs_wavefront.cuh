@@ -264,7 +264,10 @@ __device__ __forceinline__ void shade(const Scenes &scenes, const WfBuffers &b, 
                                       float4 *radiance) {
     const uint32_t n = b.count[kWfClass + cur * kWfClasses + C];
     const uint32_t *q = b.tq + static_cast<size_t>(C) * b.capacity;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    for (uint32_t first = blockIdx.x * blockDim.x; first < n; first += gridDim.x * blockDim.x) {
+        if constexpr (C == kWfClassPrincipled) __syncthreads();
+        const uint32_t i = first + threadIdx.x;
+        if (i >= n) continue;
         const uint32_t slot = q[i];
         PathState<N> ps;
         const uint32_t scene = load<N>(scenes, b, slot, ps);

@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(128, traverse_blocks(L)) k_wf_trace(const __gr
 
 // Shading of class C (0: paths that end, 1 + MaterialType: hits of that material).
 template <int N, uint32_t C>
-__global__ void __launch_bounds__(128) k_wf_shade(const __grid_constant__ DeviceScene s,
+__global__ void __launch_bounds__(shade_threads(C)) k_wf_shade(const __grid_constant__ DeviceScene s,
                                                   const __grid_constant__ WfBuffers b, uint32_t cur, uint64_t base,
                                                   float4 *radiance) {
     wf::shade<N, C>(OneScene{&s}, b, cur, base, radiance);
@@ -155,15 +155,15 @@ __global__ void __launch_bounds__(256) k_bin_scatter(const uint32_t *len, const 
 
 namespace {
 
-// Resident blocks of 128 threads per SM for each kernel, per device.
+// Resident blocks of `threads` threads per SM for each kernel, per device.
 template <typename K>
-cudaError_t resident_grid(K kernel, int dev, std::atomic<int> &cache, unsigned *grid) {
+cudaError_t resident_grid(K kernel, int dev, std::atomic<int> &cache, unsigned *grid, int threads = 128) {
     int g = cache.load();
     if (g == 0) {
         int sms = 0, per_sm = 0;
         cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return e;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0);
         if (e != cudaSuccess) return e;
         g = sms * std::max(per_sm, 1);
         cache.store(g);
@@ -179,14 +179,14 @@ struct ShadeGrids {
 template <int N, uint32_t C>
 cudaError_t shade_grid(int dev, ShadeGrids &sg) {
     static std::atomic<int> cache[64];
-    return resident_grid(k_wf_shade<N, C>, dev, cache[dev], &sg.g[C]);
+    return resident_grid(k_wf_shade<N, C>, dev, cache[dev], &sg.g[C], shade_threads(C));
 }
 
 template <int N, uint32_t C>
 void launch_shade(const ShadeGrids &sg, uint32_t mask, const DeviceScene &s, const WfBuffers &b, uint32_t cur,
                   uint64_t base, float4 *radiance, cudaStream_t st, unsigned &n_launch) {
     if (!((mask >> C) & 1u)) return;
-    k_wf_shade<N, C><<<sg.g[C], 128, 0, st>>>(s, b, cur, base, radiance);
+    k_wf_shade<N, C><<<sg.g[C], shade_threads(C), 0, st>>>(s, b, cur, base, radiance);
     ++n_launch;
 }
 
