@@ -376,8 +376,16 @@ namespace {
 // Upper bound on paths per megakernel launch; sizes the radiance scratch
 // (16 bytes per path).
 constexpr uint64_t kMaxPathsPerLaunch = 1ull << 26;
-// Path slots of one wavefront wave (208 B each: 832 MiB).
-constexpr uint64_t kWfWaveSlots = 1ull << 22;
+// Path slots of one wavefront wave of vs_render (208 B each: 3.25 GiB).  Every
+// wave ends in bounces of few paths that last as long as their slowest warps
+// (about 2 ms over the 16 bounces of the large scene), so waves are large:
+// 8.4 M paths of that scene took 26.2 ms in two waves and 22.5 ms in one.
+constexpr uint64_t kWfWaveSlots = 1ull << 24;
+// Where device memory is short the waves shrink, to this at the least.
+constexpr uint64_t kWfMinWaveSlots = 1ull << 22;
+// Pixels up to which real-time and cached frames run in wavefront form (one
+// path slot per pixel).
+constexpr uint64_t kWfFramePixels = 1ull << 22;
 
 int fail(const vs_context *ctx, int code, const std::string &msg) {
     if (ctx) {
@@ -838,10 +846,17 @@ int vs_render(vs_scene *s, uint32_t frame_begin, uint32_t frame_count, int film_
         !small && (s->schedule == VS_SCHEDULE_WAVEFRONT || s->schedule == VS_SCHEDULE_WAVEFRONT_BINNED);
     if (!wavefront && has_mix(s->host))
         return fail(ctx, VS_E_UNSUPPORTED, "mix / add materials render with the wavefront schedules only");
-    if (wavefront)
-        VS_CUDA(s->wf.ensure(static_cast<uint32_t>(std::min<uint64_t>(frames_per_chunk * npix, kWfWaveSlots)),
-                             s->schedule == VS_SCHEDULE_WAVEFRONT_BINNED),
-                "wavefront slots alloc");
+    if (wavefront) {
+        uint64_t slots = std::min<uint64_t>(frames_per_chunk * npix, kWfWaveSlots);
+        cudaError_t e;
+        while ((e = s->wf.ensure(static_cast<uint32_t>(slots), s->schedule == VS_SCHEDULE_WAVEFRONT_BINNED)) ==
+                   cudaErrorMemoryAllocation &&
+               slots > kWfMinWaveSlots) {
+            (void)cudaGetLastError();
+            slots = std::max(slots / 2, kWfMinWaveSlots);
+        }
+        VS_CUDA(e, "wavefront slots alloc");
+    }
     DeviceScene dv = s->device_view();
     auto timed_event = [&](std::vector<cudaEvent_t> &v) -> cudaError_t {
         cudaEvent_t e;
@@ -1272,7 +1287,7 @@ int restir_frame_locked(vs_scene *s, uint32_t frame_index, uint32_t film_index, 
     if (s->timing) VS_CUDA(timed_event(s->ev_render), "timing event");
     unsigned n = 0;
     const uint64_t rt_npix = static_cast<uint64_t>(p.width) * p.height;
-    const bool wavefront = s->schedule == VS_SCHEDULE_WAVEFRONT && rt_npix <= kWfWaveSlots;
+    const bool wavefront = s->schedule == VS_SCHEDULE_WAVEFRONT && rt_npix <= kWfFramePixels;
     WfBuffers wfv{};
     if (wavefront) {
         VS_CUDA(s->wf.ensure(static_cast<uint32_t>(rt_npix), false), "wavefront slots alloc");
@@ -1333,7 +1348,7 @@ int restir_prepare_locked(vs_scene *s) {
     rc = rt_ensure(s, ctx->stream);
     if (rc != VS_OK) return rc;
     const uint64_t npix = static_cast<uint64_t>(s->host.cam.width) * s->host.cam.height;
-    if (s->schedule == VS_SCHEDULE_WAVEFRONT && npix <= kWfWaveSlots) {
+    if (s->schedule == VS_SCHEDULE_WAVEFRONT && npix <= kWfFramePixels) {
         VS_CUDA(s->wf.ensure(static_cast<uint32_t>(npix), false), "wavefront slots alloc");
         VS_CUDA(s->radiance.alloc(npix), "radiance alloc");
     }
@@ -1823,7 +1838,7 @@ int vs_render_cached(vs_scene *s, vs_cache *c, uint32_t frame_begin, uint32_t fr
     p.query_depth = 2;
     p.suffix_depth = 2;
     // Wavefront frames need one path slot per pixel.
-    const bool wavefront = s->schedule == VS_SCHEDULE_WAVEFRONT && npix <= kWfWaveSlots;
+    const bool wavefront = s->schedule == VS_SCHEDULE_WAVEFRONT && npix <= kWfFramePixels;
     if (wavefront) {
         VS_CUDA(s->wf.ensure(npix, false), "wavefront slots alloc");
         VS_CUDA(s->radiance.alloc(npix), "radiance alloc");
