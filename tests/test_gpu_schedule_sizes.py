@@ -1,0 +1,90 @@
+"""vs_render's default schedule on both sides of the size where it changes from
+the persistent megakernel to wavefront passes, and across waves: the film is
+the same bits as from schedules that take one form at every size (the binned
+wavefront, the one-path-per-thread grid)."""
+import numpy as np
+import pytest
+
+from vision_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+# Paths up to which the megakernel renders, per bounce of depth (at most 16).
+DIFFUSE, OTHER = 8192, 1536
+
+
+def _films(vb, ctx, sc, frames, schedules, fp64=False):
+    s = vb.Scene(ctx, sc).build_accel()
+    out = []
+    for schedule in schedules:
+        s.set_schedule(schedule)
+        s.render(0, frames, fp64=fp64)
+        out.append((s.film(), s.film(vb.FILM_SUM64) if fp64 else None))
+    return out
+
+
+ROOMS = {
+    'box': (scenes.box_room, DIFFUSE), 'material': (scenes.material_room, OTHER),
+    'substrate': (scenes.substrate_room, OTHER), 'plastic': (scenes.plastic_room, OTHER),
+    'principled': (scenes.principled_room, OTHER), 'metallic': (scenes.metallic_room, OTHER),
+    'point': (scenes.point_light_room, DIFFUSE),
+}
+
+
+@pytest.mark.parametrize('depth', [1, 2, 8])
+@pytest.mark.parametrize('room', sorted(ROOMS))
+def test_film_on_both_sides_of_the_line(vb, gpu_ctx, room, depth):
+    make, per_depth = ROOMS[room]
+    line = min(depth, 16) * per_depth
+    w = 97
+    h = -(-line // (4 * w))
+    sc = make(width=w, height=h, max_depth=depth, dimension=3 + depth % 2)
+    for frames in (3, 4, 5):  # below, just above and above the line
+        (grid, _), (film, _) = _films(vb, gpu_ctx, sc, frames, ['grid', 'wavefront'])
+        assert np.array_equal(grid, film), (frames, w * h * frames, line)
+        assert film[..., :3].max() > 0.0
+
+
+@pytest.mark.parametrize('dimension', [1, 2, 3, 4])
+def test_environment_scene_in_wavefront_form(vb, gpu_ctx, dimension):
+    sc = scenes.large_scene(width=120, height=101, max_depth=12, subdivisions=3, grid=40, tiles=4, sky_width=256,
+                            sky_height=128, dimension=dimension)
+    assert 120 * 101 * 3 > 12 * OTHER
+    # (At one wavelength the megakernel rounds the microfacet lobes differently.)
+    others = ['wavefront_binned'] if dimension == 1 else ['wavefront_binned', 'grid', 'persistent']
+    for frames in (1, 3):
+        films = _films(vb, gpu_ctx, sc, frames, ['wavefront'] + others, fp64=True)
+        for film, sums in films[1:]:
+            assert np.array_equal(films[0][0], film)
+            assert np.array_equal(films[0][1], sums)
+
+
+def test_two_level_scene_in_wavefront_form(vb, gpu_ctx):
+    sc = scenes.instanced_scene(width=150, height=110, copies=9, subdivisions=4, patch=30, max_depth=10)
+    sc['render_setting']['instancing'] = True
+    (grid, _), (film, _) = _films(vb, gpu_ctx, sc, 2, ['grid', 'wavefront'])
+    assert 150 * 110 * 2 > 10 * OTHER
+    assert np.array_equal(grid, film)
+
+
+@pytest.mark.parametrize('frames', [1, 2])
+@pytest.mark.parametrize('room', sorted(ROOMS))
+def test_rgb_spectrum(vb, gpu_ctx, room, frames):
+    sc = ROOMS[room][0](width=160, height=100)
+    sc.pop('spectrum')
+    (binned, _), (film, _) = _films(vb, gpu_ctx, sc, frames, ['wavefront_binned', 'wavefront'])
+    assert np.array_equal(binned, film)
+
+
+@pytest.mark.parametrize('room', sorted(ROOMS))
+def test_one_wavelength(vb, gpu_ctx, room):
+    sc = ROOMS[room][0](width=90, height=60, dimension=1)
+    (binned, _), (film, _) = _films(vb, gpu_ctx, sc, 1, ['wavefront_binned', 'wavefront'])
+    assert np.array_equal(binned, film)
+
+
+def test_film_across_waves(vb, gpu_ctx):
+    # 17 x 2^20 paths: one full wave of 2^24 path slots and a second, smaller one.
+    sc = scenes.box_room(width=1024, height=1024, max_depth=2)
+    (grid, _), (film, _) = _films(vb, gpu_ctx, sc, 17, ['grid', 'wavefront'])
+    assert np.array_equal(grid, film)

@@ -439,11 +439,15 @@ uint32_t shading_classes(const HostScene &h) {
 // or glass and metal, depth 8, 739 / 378 and 1053 / 464 at 4,096 paths,
 // 768 / 882 and 1078 / 1081 at 16,384; the large scene, depth 16, 3145 / 1485
 // at 16,384, 3705 / 3049 at 65,536 and 4473 / 8245 at 262,144.  The wavefront's
-// cost grows with the depth until roulette has ended most paths.  (Mix
-// materials render in wavefront form only.)
+// cost grows with the depth until roulette has ended most paths.
+//
+// Only where the two give the same bits: at one wavelength, and under the RGB
+// spectrum, the compiler rounds some microfacet products differently in the
+// two forms.  (Mix materials render in wavefront form only.)
 bool small_render(const HostScene &h, uint64_t paths) {
     if (has_mix(h)) return false;
     const bool diffuse = (shading_classes(h) & ~(1u | (1u << (1u + kMatDiffuse)))) == 0u;
+    if (!diffuse && (h.ip.srgb || h.ip.spectrum_dim < 2u)) return false;
     return paths <= std::min<uint64_t>(h.ip.max_depth, 16u) * (diffuse ? 8192u : 1536u);
 }
 
