@@ -473,8 +473,8 @@ def run_plain(args, w, rank, world, local_rank, dist):
                      'traffic_source': 'ncu dram bytes per path of the committed profile (all kernels of the '
                                        'schedule for one render) x paths per launch',
                      'kernel': {'persistent': 'k_render_regen', 'grid': 'k_render',
-                                'wavefront': 'wavefront (k_wf_extend, k_wf_shade, k_wf_shadow)',
-                                'wavefront_binned': 'wavefront (k_wf_extend, k_wf_shade, k_wf_shadow; binned rays)'}[
+                                'wavefront': 'wavefront (k_wf_trace, k_wf_shade)',
+                                'wavefront_binned': 'wavefront (k_wf_trace, k_wf_shade; binned rays)'}[
                                     args.schedule],
                      'bytes_per_path': bytes_per_path,
                      'per_path': {'segments': segs / paths_per_step, 'nodes': nodes / paths_per_step,
