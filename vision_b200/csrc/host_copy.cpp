@@ -14,11 +14,11 @@ namespace vs {
 namespace {
 constexpr size_t kSlots = 8;
 constexpr size_t kChunk = 512u << 10;
-// Below this the threads' wake-up costs what they save.  Measured on 16 cores,
-// one thread / several: 1024 x 1024 float film (17 MB) 2.17 / 1.09 ms, 1080p
-// float film (33 MB) 4.08 / 2.47 ms, 1080p display image (8.3 MB)
-// 1.11 / 0.56 ms; 4 MB 0.62 / 0.69 ms, 1.4 MB 0.29 / 0.36 ms.
-constexpr size_t kMinBytes = 6u << 20;
+// Below this the threads' wake-up costs what they save.  Film downloads after a
+// render, measured on 16 cores, one thread / several: 1.05 MB 0.24 / 0.13 to
+// 0.27 ms, 3.2 MB 0.57 / 0.35 to 0.47, 4.9 MB 0.82 / 0.38, 17 MB 2.17 / 1.09,
+// 33 MB 4.08 / 2.47.
+constexpr size_t kMinBytes = 1u << 20;
 constexpr unsigned kMaxHelpers = 3;
 }  // namespace
 
