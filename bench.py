@@ -83,7 +83,8 @@ NCU_TRAFFIC_PER_PATH = {('large_scene', 'persistent'): 383.6e6 / 2097152,
 # workload's 2-spp case (the binding measure of the L1/L2-resident traversal).
 NCU_ISSUE = {('large_scene', 'wavefront'): {
     'issue_active': 0.652, 'threads_per_inst': 12.95,
-    'issue_source': 'ncu sm__inst_issued / smsp__thread_inst_executed_per_inst_executed of k_wf_extend '
+    'issue_source': 'ncu sm__inst_issued / smsp__thread_inst_executed_per_inst_executed of k_wf_extend, '
+                    'the closest-hit pass before path and shadow rays shared k_wf_trace '
                     '(profiles/k_wf_extend_large_scene.md)'}}
 
 # Algorithmic bytes per pixel-frame of the ReSTIR frame, from the record sizes
