@@ -102,6 +102,36 @@ def test_degenerate_rays_bit_exact(vb, gpu_ctx, offset, soup):
     assert np.array_equal(s.trace_any(rays) != 0, ~miss)
 
 
+@pytest.mark.parametrize('offset, size, spread', [(1e8, 3e2, 3e3), (5e8, 3e3, 2e4), (3e9, 2e4, 1e5)])
+def test_axis_parallel_rays_far_from_the_origin(vb, gpu_ctx, offset, size, spread):
+    # A direction component of zero times a coordinate above 3.4e8 overflows
+    # in a box test that multiplies by the reciprocal.
+    rng = np.random.default_rng(1)
+    P = (rng.random((300, 1, 3)) * spread + size * rng.normal(size=(300, 3, 3)) + offset).astype(np.float32)
+    sc = scenes.box_room(width=4, height=4)
+    sc['shapes'].append({'type': 'mesh', 'name': 'soup', 'param': {
+        'positions': P.reshape(-1).tolist(), 'indices': list(range(900)), 'material': 'Floor'}})
+    s = vb.Scene(gpu_ctx, sc).build_accel()
+    pos, idx = s.export('pos', np.float32), s.export('idx', np.uint32)
+    tris = pos.reshape(-1, 3)[idx.reshape(-1, 3)]
+    n = 4096
+    rays = np.zeros((n, 8), np.float32)
+    axis, sign = rng.integers(0, 3, n), rng.choice([-1.0, 1.0], n)
+    rays[np.arange(n), 4 + axis] = sign
+    rays[:, 0:3] = tris[rng.integers(len(tris) - 300, len(tris), n)].mean(1) - 2 * spread * rays[:, 4:7]
+    negative = (rays[:, 4:7] == 0.0) & (rng.random((n, 1)) < 0.5)
+    rays[:, 4:7][negative] = -0.0
+    rays[:, 7] = 1e30
+    prim, uvt = _brute_force(tris, rays)
+    hits, t = s.trace_closest(rays)
+    hit = prim != 0xffffffff
+    assert hit.mean() > 0.9
+    assert np.array_equal(hits[:, 1], prim)
+    assert np.array_equal(hits[hit, 2:], uvt[hit, :2].copy().view(np.uint32))
+    assert np.array_equal(t[hit], uvt[hit, 2])
+    assert np.array_equal(s.trace_any(rays) != 0, hit)
+
+
 @pytest.mark.parametrize('n', [1, 31, 33, 127, 129, 5000, 300001])
 def test_batch_sizes_bit_exact(vb, gpu_ctx, n):
     s = vb.Scene(gpu_ctx, scenes.box_room()).build_accel()

@@ -337,12 +337,18 @@ struct RayPre {
 // `bound`: the largest coordinate magnitude, per axis, of the BVH's boxes.
 //
 // The box distances of intersect_children are q * (2^e / d) + ((p - o) / d),
-// the second term as p / d + (-o / d).  Its roundings, those of the quantised
-// planes and those of the triangle test are each at most a few 2^-24 of
-// (|o| + |plane|) / |d|; cn and cf move every near plane down and every far
-// plane up by 2^-21 of that, so a box is entered whenever the float triangle
-// test can accept one of its triangles.  (1 / d is an approximation, good to
-// 2 ulp, for the same reason; the shear factors are exactly rounded.)
+// the second term as p / d + (-o / d).  In units of 2^-24 (|o| + |plane|) / |d|
+// the reciprocal (good to 2 ulp) costs them up to 4, their own roundings up to
+// 6 and the triangle test's vertex differences and shear up to 4.  cn and cf
+// move every near plane down and every far plane up by 16 of these units, so a
+// box is entered whenever the float triangle test can accept one of its
+// triangles.  Measured against rays aimed at the corners of axis-aligned
+// triangles, with the reciprocal off by 2 ulp: 4 units lose 0.8 % of the hits,
+// 6 units 2 in a million, 8 units none of 47 million.
+// The margin is taken of |o / d| as it was computed, so that it is infinite
+// wherever that overflows (a zero direction component, |o| above 3.4e8): the
+// planes of the axis are then infinite or NaN on the side that keeps the box
+// (a NaN is dropped by the minima and maxima).
 __device__ __forceinline__ RayPre precompute_ray(f3 o, f3 d, f3 bound) {
     RayPre r;
     r.wo = o;
@@ -351,10 +357,10 @@ __device__ __forceinline__ RayPre precompute_ray(f3 o, f3 d, f3 bound) {
     r.inv_d = {__fdividef(1.0f, fabsf(d.x) > tiny ? d.x : copysignf(tiny, d.x)),
                __fdividef(1.0f, fabsf(d.y) > tiny ? d.y : copysignf(tiny, d.y)),
                __fdividef(1.0f, fabsf(d.z) > tiny ? d.z : copysignf(tiny, d.z))};
-    const float k = 1.0f / 2097152.0f;
+    const float k = 1.0f / 1048576.0f;
     const f3 b = {-o.x * r.inv_d.x, -o.y * r.inv_d.y, -o.z * r.inv_d.z};
-    const f3 e = {k * (bound.x + fabsf(o.x)) * fabsf(r.inv_d.x), k * (bound.y + fabsf(o.y)) * fabsf(r.inv_d.y),
-                  k * (bound.z + fabsf(o.z)) * fabsf(r.inv_d.z)};
+    const f3 e = {k * fmaf(bound.x, fabsf(r.inv_d.x), fabsf(b.x)), k * fmaf(bound.y, fabsf(r.inv_d.y), fabsf(b.y)),
+                  k * fmaf(bound.z, fabsf(r.inv_d.z), fabsf(b.z))};
     r.cn = b - e;
     r.cf = b + e;
     float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
