@@ -553,10 +553,11 @@ struct Bsdf {
             else wi = substrate_sample(wo, smp.next2());
         } else if (has_mat<M>(kMatPrincipled) && type == kMatPrincipled) {
             // LobeSet::sample_wi_impl (lobe.cpp:598-627): 1D lobe choice, an
-            // unused 2D draw, then the chosen lobe's own draws.
+            // unused 2D draw, then the chosen lobe's own draws.  A draw of zero
+            // takes the first lobe of the set.
             float uc = smp.next();
             (void)smp.next2();
-            int strategy = 0;
+            int strategy = -1;
             float sum = 0.0f;
             const float ws[6] = {w_sheen, w_coat, w_metal, w_trans, w_spec, w_diff};
             const bool present[6] = {w_sheen > 0.0f, w_coat > 0.0f, w_metal > 0.0f, has_trans, w_spec > 0.0f,
@@ -564,7 +565,7 @@ struct Bsdf {
 #pragma unroll
             for (int i = 0; i < 6; ++i) {
                 if (!present[i]) continue;
-                strategy = uc > sum ? i : strategy;
+                strategy = uc > sum || strategy < 0 ? i : strategy;
                 sum += ws[i];
             }
             wi = sample_principled_lobe(strategy, wo, smp, valid);
@@ -861,7 +862,7 @@ struct MixBsdf {
         const f3 wo = c[0].frame.to_local(wo_w);
         const float uc = smp.next();
         (void)smp.next2();
-        int child = 0, lobe = -1;
+        int child = -1, lobe = -1;
         float sum = 0.0f;
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
@@ -873,14 +874,14 @@ struct MixBsdf {
 #pragma unroll
                 for (int i = 0; i < 6; ++i) {
                     if (!present[i]) continue;
-                    if (uc > sum) {
+                    if (uc > sum || child < 0) {
                         child = k;
                         lobe = i;
                     }
                     sum += ws[i] * sw[k];
                 }
             } else {
-                if (uc > sum) {
+                if (uc > sum || child < 0) {
                     child = k;
                     lobe = -1;
                 }
@@ -888,7 +889,7 @@ struct MixBsdf {
             }
         }
         bool valid = true;
-        const Bsdf<N> &b = c[child];
+        const Bsdf<N> &b = c[child == 1 ? 1 : 0];
         const f3 wi = lobe < 0 ? b.sample_dir(wo, smp, valid) : b.sample_principled_lobe(lobe, wo, smp, valid);
         BsdfSample<N> bs;
         bs.eta = 1.0f;
