@@ -202,12 +202,10 @@ int vs_render(vs_scene *scene, uint32_t frame_begin, uint32_t frame_count, int f
  * VS_SCHEDULE_GRID: one path per thread over a grid that covers all paths of
  * a launch.  VS_SCHEDULE_PERSISTENT: one resident wave of warps that keep 32
  * paths in flight each and refill the lanes of finished paths after every
- * bounce (path regeneration).  VS_SCHEDULE_WAVEFRONT (the default): waves of
- * up to 16,777,216 paths whose bounces run as separate kernels (traversal,
- * shading sorted by material) over path state in device memory (208 bytes per
- * path slot, allocated on first use; smaller waves where memory is short);
- * renders of so few paths that the passes' fixed cost decides run as
- * VS_SCHEDULE_PERSISTENT does. */
+ * bounce (path regeneration).  VS_SCHEDULE_WAVEFRONT: waves of up to
+ * 16,777,216 paths whose bounces run as separate kernels (traversal, shading
+ * sorted by material) over path state in device memory (208 bytes per path
+ * slot, allocated on first use; smaller waves where memory is short). */
 #define VS_SCHEDULE_GRID 0
 #define VS_SCHEDULE_PERSISTENT 1
 #define VS_SCHEDULE_WAVEFRONT 2
@@ -217,6 +215,10 @@ int vs_render(vs_scene *scene, uint32_t frame_begin, uint32_t frame_count, int f
  * three small kernels), so that each warp traces rays that start close
  * together and visit children in the same order; 12 more bytes per slot. */
 #define VS_SCHEDULE_WAVEFRONT_BINNED 3
+/* The default: VS_SCHEDULE_PERSISTENT for renders of so few paths that the
+ * wavefront passes' fixed cost decides, VS_SCHEDULE_WAVEFRONT otherwise (and
+ * for real-time and cached frames). */
+#define VS_SCHEDULE_AUTO 4
 int vs_render_schedule_set(vs_scene *scene, int schedule);
 
 /* Waits for all work queued on the scene's stream. */

@@ -1,7 +1,7 @@
-"""vs_render's default schedule on both sides of the size where it changes from
-the persistent megakernel to wavefront passes, and across waves: the film is
-the same bits as from schedules that take one form at every size (the binned
-wavefront, the one-path-per-thread grid)."""
+"""vs_render's default schedule ('auto') on both sides of the size where it
+changes from the persistent megakernel to wavefront passes, and wavefront
+passes across waves: the film is the same bits as from schedules that take one
+form at every size."""
 import numpy as np
 import pytest
 
@@ -40,9 +40,27 @@ def test_film_on_both_sides_of_the_line(vb, gpu_ctx, room, depth):
     h = -(-line // (4 * w))
     sc = make(width=w, height=h, max_depth=depth, dimension=3 + depth % 2)
     for frames in (3, 4, 5):  # below, just above and above the line
-        (grid, _), (film, _) = _films(vb, gpu_ctx, sc, frames, ['grid', 'wavefront'])
+        (grid, _), (waves, _), (film, _) = _films(vb, gpu_ctx, sc, frames, ['grid', 'wavefront', 'auto'])
         assert np.array_equal(grid, film), (frames, w * h * frames, line)
+        assert np.array_equal(waves, film), (frames, w * h * frames, line)
         assert film[..., :3].max() > 0.0
+
+
+@pytest.mark.parametrize('room', ['box', 'principled'])
+def test_named_schedules_keep_their_form(vb, gpu_ctx, room):
+    # The grid and the megakernel are one kernel and the film pass; wavefront
+    # passes are several for each bounce, at any size.
+    s = vb.Scene(gpu_ctx, ROOMS[room][0](width=16, height=16, max_depth=4)).build_accel()
+    count = {}
+    for schedule in (None, 'grid', 'persistent', 'wavefront', 'wavefront_binned', 'auto'):
+        if schedule:
+            s.set_schedule(schedule)
+        n = vb.launch_count()
+        s.render(0, 1)
+        count[schedule] = vb.launch_count() - n
+    assert count[None] == count['auto'] == count['persistent'] == count['grid'] == 2
+    assert count['wavefront'] >= 2 + 2 * 4
+    assert count['wavefront_binned'] > count['wavefront']
 
 
 @pytest.mark.parametrize('dimension', [1, 2, 3, 4])
@@ -51,7 +69,7 @@ def test_environment_scene_in_wavefront_form(vb, gpu_ctx, dimension):
                             sky_height=128, dimension=dimension)
     assert 120 * 101 * 3 > 12 * OTHER
     # (At one wavelength the megakernel rounds the microfacet lobes differently.)
-    others = ['wavefront_binned'] if dimension == 1 else ['wavefront_binned', 'grid', 'persistent']
+    others = ['wavefront_binned', 'auto'] + ([] if dimension == 1 else ['grid', 'persistent'])
     for frames in (1, 3):
         films = _films(vb, gpu_ctx, sc, frames, ['wavefront'] + others, fp64=True)
         for film, sums in films[1:]:
@@ -62,9 +80,10 @@ def test_environment_scene_in_wavefront_form(vb, gpu_ctx, dimension):
 def test_two_level_scene_in_wavefront_form(vb, gpu_ctx):
     sc = scenes.instanced_scene(width=150, height=110, copies=9, subdivisions=4, patch=30, max_depth=10)
     sc['render_setting']['instancing'] = True
-    (grid, _), (film, _) = _films(vb, gpu_ctx, sc, 2, ['grid', 'wavefront'])
+    (grid, _), (film, _), (auto, _) = _films(vb, gpu_ctx, sc, 2, ['grid', 'wavefront', 'auto'])
     assert 150 * 110 * 2 > 10 * OTHER
     assert np.array_equal(grid, film)
+    assert np.array_equal(grid, auto)
 
 
 @pytest.mark.parametrize('frames', [1, 2])
@@ -72,15 +91,17 @@ def test_two_level_scene_in_wavefront_form(vb, gpu_ctx):
 def test_rgb_spectrum(vb, gpu_ctx, room, frames):
     sc = ROOMS[room][0](width=160, height=100)
     sc.pop('spectrum')
-    (binned, _), (film, _) = _films(vb, gpu_ctx, sc, frames, ['wavefront_binned', 'wavefront'])
+    (binned, _), (film, _), (auto, _) = _films(vb, gpu_ctx, sc, frames, ['wavefront_binned', 'wavefront', 'auto'])
     assert np.array_equal(binned, film)
+    assert np.array_equal(auto, film)
 
 
 @pytest.mark.parametrize('room', sorted(ROOMS))
 def test_one_wavelength(vb, gpu_ctx, room):
     sc = ROOMS[room][0](width=90, height=60, dimension=1)
-    (binned, _), (film, _) = _films(vb, gpu_ctx, sc, 1, ['wavefront_binned', 'wavefront'])
+    (binned, _), (film, _), (auto, _) = _films(vb, gpu_ctx, sc, 1, ['wavefront_binned', 'wavefront', 'auto'])
     assert np.array_equal(binned, film)
+    assert np.array_equal(auto, film)
 
 
 def test_film_across_waves(vb, gpu_ctx):

@@ -88,7 +88,9 @@ struct vs_scene {
     DevBuf<float4> radiance;
     // Path counter of the persistent (regenerating) megakernel.
     DevBuf<unsigned long long> path_counter;
-    int schedule = VS_SCHEDULE_WAVEFRONT;
+    int schedule = VS_SCHEDULE_AUTO;
+    // Whether real-time and cached frames run as wavefront passes.
+    bool wavefront_frames() const { return schedule == VS_SCHEDULE_AUTO || schedule == VS_SCHEDULE_WAVEFRONT; }
     // Path slots of the wavefront schedule.
     struct WfBufs {
         DevBuf<float4> o, d, tp, lam, pdf, L, sh_o, sh_d, sh_c;
@@ -429,8 +431,8 @@ uint32_t shading_classes(const HostScene &h) {
     return m;
 }
 
-// Whether vs_render's wavefront schedule renders `paths` paths with the
-// persistent megakernel instead (the same films, bit for bit).  A wavefront
+// Whether VS_SCHEDULE_AUTO renders `paths` paths with the persistent
+// megakernel instead of wavefront passes (the same films, bit for bit).  A wavefront
 // bounce is a traversal pass and one shading pass per class, each of which
 // lasts as long as its slowest warp however few paths it has; the megakernel
 // has no such steps but runs all materials' code at low occupancy.  Measured
@@ -843,17 +845,19 @@ int vs_render(vs_scene *s, uint32_t frame_begin, uint32_t frame_count, int film_
     if (frames_per_chunk == 0) return fail(ctx, VS_E_RANGE, "resolution above the per-launch path limit");
     if (frames_per_chunk > frame_count) frames_per_chunk = frame_count;
     VS_CUDA(s->radiance.alloc(static_cast<size_t>(frames_per_chunk * npix)), "radiance alloc");
-    const bool small = s->schedule == VS_SCHEDULE_WAVEFRONT && small_render(s->host, frames_per_chunk * npix);
-    const bool persistent = s->schedule == VS_SCHEDULE_PERSISTENT || small;
+    int schedule = s->schedule;
+    if (schedule == VS_SCHEDULE_AUTO)
+        schedule = small_render(s->host, frames_per_chunk * npix) ? VS_SCHEDULE_PERSISTENT : VS_SCHEDULE_WAVEFRONT;
+    const bool persistent = schedule == VS_SCHEDULE_PERSISTENT;
     if (persistent) VS_CUDA(s->path_counter.alloc(1), "path counter alloc");
-    const bool wavefront =
-        !small && (s->schedule == VS_SCHEDULE_WAVEFRONT || s->schedule == VS_SCHEDULE_WAVEFRONT_BINNED);
+    const bool binned = schedule == VS_SCHEDULE_WAVEFRONT_BINNED;
+    const bool wavefront = schedule == VS_SCHEDULE_WAVEFRONT || binned;
     if (!wavefront && has_mix(s->host))
         return fail(ctx, VS_E_UNSUPPORTED, "mix / add materials render with the wavefront schedules only");
     if (wavefront) {
         uint64_t slots = std::min<uint64_t>(frames_per_chunk * npix, kWfWaveSlots);
         cudaError_t e;
-        while ((e = s->wf.ensure(static_cast<uint32_t>(slots), s->schedule == VS_SCHEDULE_WAVEFRONT_BINNED)) ==
+        while ((e = s->wf.ensure(static_cast<uint32_t>(slots), binned)) ==
                    cudaErrorMemoryAllocation &&
                slots > kWfMinWaveSlots) {
             (void)cudaGetLastError();
@@ -875,8 +879,7 @@ int vs_render(vs_scene *s, uint32_t frame_begin, uint32_t frame_count, int film_
         if (wavefront) {
             unsigned n = 0;
             VS_CUDA(launch_render_wavefront(dv, frame_begin + f, fc, s->radiance.ptr,
-                                            s->schedule == VS_SCHEDULE_WAVEFRONT_BINNED ? s->wf.view_binned()
-                                                                                        : s->wf.view(),
+                                            binned ? s->wf.view_binned() : s->wf.view(),
                                             shading_classes(s->host), st, &n),
                     "wavefront render");
             add_launches(n);
@@ -908,9 +911,9 @@ int vs_render(vs_scene *s, uint32_t frame_begin, uint32_t frame_count, int film_
 int vs_render_schedule_set(vs_scene *s, int schedule) {
     if (!s) return VS_E_INVALID;
     if (schedule != VS_SCHEDULE_GRID && schedule != VS_SCHEDULE_PERSISTENT && schedule != VS_SCHEDULE_WAVEFRONT &&
-        schedule != VS_SCHEDULE_WAVEFRONT_BINNED)
+        schedule != VS_SCHEDULE_WAVEFRONT_BINNED && schedule != VS_SCHEDULE_AUTO)
         return fail(s->ctx, VS_E_INVALID,
-                    "schedule must be VS_SCHEDULE_GRID, _PERSISTENT, _WAVEFRONT or _WAVEFRONT_BINNED");
+                    "schedule must be VS_SCHEDULE_GRID, _PERSISTENT, _WAVEFRONT, _WAVEFRONT_BINNED or _AUTO");
     std::lock_guard<std::mutex> lock(s->mu);
     s->schedule = schedule;
     return VS_OK;
@@ -1291,7 +1294,7 @@ int restir_frame_locked(vs_scene *s, uint32_t frame_index, uint32_t film_index, 
     if (s->timing) VS_CUDA(timed_event(s->ev_render), "timing event");
     unsigned n = 0;
     const uint64_t rt_npix = static_cast<uint64_t>(p.width) * p.height;
-    const bool wavefront = s->schedule == VS_SCHEDULE_WAVEFRONT && rt_npix <= kWfFramePixels;
+    const bool wavefront = s->wavefront_frames() && rt_npix <= kWfFramePixels;
     WfBuffers wfv{};
     if (wavefront) {
         VS_CUDA(s->wf.ensure(static_cast<uint32_t>(rt_npix), false), "wavefront slots alloc");
@@ -1352,7 +1355,7 @@ int restir_prepare_locked(vs_scene *s) {
     rc = rt_ensure(s, ctx->stream);
     if (rc != VS_OK) return rc;
     const uint64_t npix = static_cast<uint64_t>(s->host.cam.width) * s->host.cam.height;
-    if (s->schedule == VS_SCHEDULE_WAVEFRONT && npix <= kWfFramePixels) {
+    if (s->wavefront_frames() && npix <= kWfFramePixels) {
         VS_CUDA(s->wf.ensure(static_cast<uint32_t>(npix), false), "wavefront slots alloc");
         VS_CUDA(s->radiance.alloc(npix), "radiance alloc");
     }
@@ -1842,7 +1845,7 @@ int vs_render_cached(vs_scene *s, vs_cache *c, uint32_t frame_begin, uint32_t fr
     p.query_depth = 2;
     p.suffix_depth = 2;
     // Wavefront frames need one path slot per pixel.
-    const bool wavefront = s->schedule == VS_SCHEDULE_WAVEFRONT && npix <= kWfFramePixels;
+    const bool wavefront = s->wavefront_frames() && npix <= kWfFramePixels;
     if (wavefront) {
         VS_CUDA(s->wf.ensure(npix, false), "wavefront slots alloc");
         VS_CUDA(s->radiance.alloc(npix), "radiance alloc");
