@@ -436,21 +436,33 @@ uint32_t shading_classes(const HostScene &h) {
 // bounce is a traversal pass and one shading pass per class, each of which
 // lasts as long as its slowest warp however few paths it has; the megakernel
 // has no such steps but runs all materials' code at low occupancy.  Measured
-// crossing points (us, wavefront / megakernel): box room of depth 8, diffuse,
-// 519 / 397 at 65,536 paths and 572 / 676 at 131,044; rooms with principled
-// or glass and metal, depth 8, 739 / 378 and 1053 / 464 at 4,096 paths,
-// 768 / 882 and 1078 / 1081 at 16,384; the large scene, depth 16, 3145 / 1485
-// at 16,384, 3705 / 3049 at 65,536 and 4473 / 8245 at 262,144.  The wavefront's
-// cost grows with the depth until roulette has ended most paths.
+// at 1,024 to 131,044 paths and depths 1, 2, 4, 8 and 16 (us, wavefront /
+// megakernel, on both sides of the lines below):
+//   diffuse rooms, depth 8: area light 398 / 280 at 49,152 paths and 415 / 414
+//   at 98,304; projectors 349 / 309 and 368 / 392 at 65,536 (the earliest
+//   crossing); 10,000 diffuse triangles under a sky 712 / 629 and 774 / 837 at
+//   98,304; depth 4: 208 / 129 at 24,576, 228 / 244 at 65,536;
+//   depth 16: projectors 676 / 529 at 98,304, 758 / 698 at 131,044;
+//   other materials, depth 8: principled 678 / 658 at 12,288 paths and 687 / 848
+//   at 16,384; glass and metal 935 / 780 and 949 / 993; image textures 738 / 469
+//   and 752 / 647 at 24,576; 0.58 M triangles 1463 / 748 and 1691 / 1905 at
+//   65,536; two levels 1147 / 686 and no crossing up to 131,044;
+//   depth 4: principled 343 / 231 at 8,192, 355 / 361 at 12,288; depth 16:
+//   1295 / 1110 at 24,576, 1320 / 1578 at 32,832.
+// The wavefront's cost grows with the depth until roulette has ended most
+// paths.
 //
-// Only where the two give the same bits: at one wavelength, and under the RGB
-// spectrum, the compiler rounds some microfacet products differently in the
-// two forms.  (Mix materials render in wavefront form only.)
+// Only where the two give the same bits, which depends on how the compiler
+// rounds shared products in either kernel: at one wavelength it rounds some
+// microfacet and environment products differently.  (Under the RGB spectrum
+// materials other than diffuse have differed in former builds; mix materials
+// render in wavefront form only.)
 bool small_render(const HostScene &h, uint64_t paths) {
     if (has_mix(h)) return false;
     const bool diffuse = (shading_classes(h) & ~(1u | (1u << (1u + kMatDiffuse)))) == 0u;
-    if (!diffuse && (h.ip.srgb || h.ip.spectrum_dim < 2u)) return false;
-    return paths <= std::min<uint64_t>(h.ip.max_depth, 16u) * (diffuse ? 8192u : 1536u);
+    if (!diffuse && h.ip.srgb) return false;
+    if (h.ip.spectrum_dim < 2u && (!diffuse || h.has_env)) return false;
+    return paths <= std::min<uint64_t>(h.ip.max_depth, 16u) * (diffuse ? 7168u : 1536u);
 }
 
 // Per instance: the world-to-object rows and (mesh root node, first
