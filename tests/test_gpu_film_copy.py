@@ -1,0 +1,58 @@
+"""Film downloads: the threaded copy into pageable memory against the direct
+copy into page-locked memory, and its cost to the host while a render is still
+running."""
+import ctypes
+import time
+
+import numpy as np
+import pytest
+import torch
+
+from vision_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+PIXELS_1MB = (1 << 20) // 16  # of a linear film: the smallest threaded copy
+CHUNK = (512 << 10) // 16
+RING = 8 * CHUNK
+
+
+def _scene(vb, ctx, width, height=1, seed=0):
+    sc = scenes.box_room(width=width, height=height, max_depth=2, sampler='pcg')
+    sc['sampler']['param']['seed'] = seed
+    return vb.Scene(ctx, sc).build_accel()
+
+
+def _download(vb, s, address, pixels, which=0):
+    s.ctx.check(vb.lib.vs_film_download(s.handle, ctypes.c_void_p(address), pixels * 16, which), 'film_download')
+
+
+@pytest.mark.parametrize('pixels', [PIXELS_1MB - 1, PIXELS_1MB, PIXELS_1MB + 1, 3 * CHUNK - 1, 3 * CHUNK + 1, RING - 1, RING,
+                                    RING + 1, RING + CHUNK, RING + CHUNK + 1, 3 * RING + 5])
+def test_threaded_copy_equals_direct_copy(vb, gpu_ctx, pixels):
+    width = pixels if pixels < 1 << 16 else next(w for w in range(1 << 15, 0, -1) if pixels % w == 0)
+    s = _scene(vb, gpu_ctx, width, pixels // width)
+    s.render(0, 1)
+    pinned = torch.empty(pixels * 4, dtype=torch.float32, pin_memory=True)
+    _download(vb, s, pinned.data_ptr(), pixels)
+    want = pinned.numpy().view(np.uint8)
+    assert want.any()
+    for misalign in (0, 1, 4):
+        buf = np.full(pixels * 16 + 64, 0xa5, np.uint8)
+        start = -buf.ctypes.data % 16 + misalign
+        _download(vb, s, buf.ctypes.data + start, pixels)
+        assert np.array_equal(buf[start:start + pixels * 16], want)
+        assert np.all(buf[:start] == 0xa5) and np.all(buf[start + pixels * 16:] == 0xa5)  # nothing written around it
+
+
+def test_download_behind_a_long_render_keeps_one_thread_busy(vb, gpu_ctx):
+    s = _scene(vb, gpu_ctx, 1024, 1024)
+    s.render(0, 1)
+    s.film()
+    s.render(0, 600)  # returns at once; hundreds of milliseconds of work
+    cpu, wall = time.process_time(), time.perf_counter()
+    s.film()
+    cpu, wall = time.process_time() - cpu, time.perf_counter() - wall
+    assert wall > 0.05
+    # The waiting thread, and the copy itself at the end; not the helpers too.
+    assert cpu < 1.7 * wall

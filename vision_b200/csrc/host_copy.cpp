@@ -25,6 +25,7 @@ constexpr unsigned kMaxHelpers = 3;
 struct HostCopy::Impl {
     uint8_t *ring = nullptr;
     cudaEvent_t ev[kSlots] = {};
+    cudaEvent_t ready = nullptr;  // the work before the copy has ended
     std::vector<std::thread> helpers;
     std::mutex one;  // one copy at a time
 
@@ -53,6 +54,7 @@ struct HostCopy::Impl {
             return e;
         }
         for (size_t i = 0; i < kSlots && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
         if (e != cudaSuccess) {
             release();
             return e;
@@ -71,6 +73,8 @@ struct HostCopy::Impl {
             if (e) cudaEventDestroy(e);
             e = nullptr;
         }
+        if (ready) cudaEventDestroy(ready);
+        ready = nullptr;
         if (ring) cudaFreeHost(ring);
         ring = nullptr;
     }
@@ -140,8 +144,13 @@ struct HostCopy::Impl {
         next = 0;
         error = 0;
         for (auto &q : queued) q = 0;
+        e = cudaEventRecord(ready, stream);
+        if (e != cudaSuccess) return e;
         for (size_t k = 0; k < std::min(chunks, kSlots); ++k)
             if (!queue(k)) break;
+        // Only this thread waits for the work before the copy (which may be a
+        // long render); the helpers start as the first chunk is on its way.
+        if (!error.load() && (e = cudaEventSynchronize(ready)) != cudaSuccess) error = e;
         {
             std::lock_guard<std::mutex> lk(mu);
             ++generation;
