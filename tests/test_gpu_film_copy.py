@@ -1,7 +1,8 @@
 """Film downloads: the threaded copy into pageable memory against the direct
-copy into page-locked memory, and its cost to the host while a render is still
-running."""
+copy into page-locked memory, its cost to the host while a render is still
+running, and renders of other scenes beside it."""
 import ctypes
+import threading
 import time
 
 import numpy as np
@@ -56,3 +57,50 @@ def test_download_behind_a_long_render_keeps_one_thread_busy(vb, gpu_ctx):
     assert wall > 0.05
     # The waiting thread, and the copy itself at the end; not the helpers too.
     assert cpu < 1.7 * wall
+
+
+def test_download_does_not_wait_for_a_later_render(vb, gpu_ctx):
+    a, b = _scene(vb, gpu_ctx, 2048, 1024, 1), _scene(vb, gpu_ctx, 512, 512, 2)
+    a.render(0, 1)
+    want = a.film()
+    b.render(0, 1500)
+    gpu_ctx.check(vb.lib.vs_synchronize(b.handle), 'synchronize')
+    t = time.perf_counter()
+    b.render(0, 1500)
+    gpu_ctx.check(vb.lib.vs_synchronize(b.handle), 'synchronize')
+    later = time.perf_counter() - t
+    a.render(0, 1)
+    a.render(1, 40)  # the download waits for these
+    got = []
+    thread = threading.Thread(target=lambda: got.append((a.film(), time.perf_counter())))
+    t = time.perf_counter()
+    thread.start()
+    time.sleep(0.002)
+    b.render(0, 1500)
+    queued = time.perf_counter() - t
+    thread.join()
+    gpu_ctx.check(vb.lib.vs_synchronize(b.handle), 'synchronize')
+    assert got[0][0].shape == want.shape
+    assert queued < 0.5 * later  # the render was queued while the download waited
+    assert got[0][1] - t < 0.7 * later
+
+
+def test_downloads_and_renders_on_several_threads(vb, gpu_ctx):
+    made = [_scene(vb, gpu_ctx, 1200, 700, k) for k in range(3)]
+    want = []
+    for s in made:
+        s.render(0, 2)
+        want.append(s.film())
+    wrong = []
+
+    def work(k):
+        for _ in range(12):
+            made[k].render(0, 2)
+            if not np.array_equal(made[k].film(), want[k]):
+                wrong.append(k)
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong

@@ -26,6 +26,9 @@ struct HostCopy::Impl {
     uint8_t *ring = nullptr;
     cudaEvent_t ev[kSlots] = {};
     cudaEvent_t ready = nullptr;  // the work before the copy has ended
+    // The chunks' own stream: the later ones are queued as slots empty, and on
+    // the caller's stream another thread's render could have come before them.
+    cudaStream_t st = nullptr;
     std::vector<std::thread> helpers;
     std::mutex one;  // one copy at a time
 
@@ -35,7 +38,6 @@ struct HostCopy::Impl {
     const uint8_t *src = nullptr;
     size_t bytes = 0, chunks = 0;
     int device = 0;
-    cudaStream_t st = nullptr;
     std::atomic<size_t> next{0};
     std::atomic<size_t> queued[kSlots];  // chunks queued into the slot so far
     std::atomic<int> error{0};
@@ -55,6 +57,7 @@ struct HostCopy::Impl {
         }
         for (size_t i = 0; i < kSlots && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
         if (e != cudaSuccess) {
             release();
             return e;
@@ -73,6 +76,8 @@ struct HostCopy::Impl {
             if (e) cudaEventDestroy(e);
             e = nullptr;
         }
+        if (st) cudaStreamDestroy(st);
+        st = nullptr;
         if (ready) cudaEventDestroy(ready);
         ready = nullptr;
         if (ring) cudaFreeHost(ring);
@@ -140,11 +145,11 @@ struct HostCopy::Impl {
         bytes = n;
         chunks = (n + kChunk - 1) / kChunk;
         device = dev;
-        st = stream;
         next = 0;
         error = 0;
         for (auto &q : queued) q = 0;
         e = cudaEventRecord(ready, stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ready, 0);
         if (e != cudaSuccess) return e;
         for (size_t k = 0; k < std::min(chunks, kSlots); ++k)
             if (!queue(k)) break;
@@ -162,7 +167,7 @@ struct HostCopy::Impl {
         cv_end.wait(lk, [&] { return running == 0; });
         if (error.load()) {
             // Nothing may still be writing the ring when the next copy starts.
-            (void)cudaStreamSynchronize(stream);
+            (void)cudaStreamSynchronize(st);
         }
         return static_cast<cudaError_t>(error.load());
     }
