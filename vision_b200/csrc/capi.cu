@@ -612,6 +612,7 @@ int vs_context_create(int device, vs_context **out) {
             delete ctx;
             return VS_E_CUDA;
         }
+        ctx->download.prepare();
     }
     *out = ctx;
     return VS_OK;

@@ -49,7 +49,6 @@ struct HostCopy::Impl {
     bool stop = false;
 
     cudaError_t init() {
-        if (ring) return cudaSuccess;
         cudaError_t e = cudaHostAlloc(reinterpret_cast<void **>(&ring), kSlots * kChunk, cudaHostAllocPortable);
         if (e != cudaSuccess) {
             ring = nullptr;
@@ -133,13 +132,6 @@ struct HostCopy::Impl {
 
     cudaError_t copy(void *d, const void *s, size_t n, int dev, cudaStream_t stream) {
         std::lock_guard<std::mutex> guard(one);
-        cudaError_t e = init();
-        if (e != cudaSuccess) {
-            // No page-locked memory to be had: the plain copy does not need it.
-            (void)cudaGetLastError();
-            e = cudaMemcpyAsync(d, s, n, cudaMemcpyDeviceToHost, stream);
-            return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
-        }
         dst = static_cast<uint8_t *>(d);
         src = static_cast<const uint8_t *>(s);
         bytes = n;
@@ -148,7 +140,7 @@ struct HostCopy::Impl {
         next = 0;
         error = 0;
         for (auto &q : queued) q = 0;
-        e = cudaEventRecord(ready, stream);
+        cudaError_t e = cudaEventRecord(ready, stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ready, 0);
         if (e != cudaSuccess) return e;
         for (size_t k = 0; k < std::min(chunks, kSlots); ++k)
@@ -186,12 +178,17 @@ struct HostCopy::Impl {
 HostCopy::HostCopy() : impl(new Impl()) {}
 HostCopy::~HostCopy() { delete impl; }
 
+void HostCopy::prepare() {
+    // Where no page-locked memory is to be had, copies go without it.
+    if (impl->init() != cudaSuccess) (void)cudaGetLastError();
+}
+
 cudaError_t HostCopy::copy(void *dst, const void *src, size_t bytes, int device, cudaStream_t st) {
     // Page-locked (or device) destinations take the copy directly.
     cudaPointerAttributes at{};
     const bool pageable = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
     (void)cudaGetLastError();
-    if (bytes < kMinBytes || !pageable) {
+    if (bytes < kMinBytes || !pageable || !impl->ring) {
         const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
         return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
     }
