@@ -203,9 +203,10 @@ int vs_render(vs_scene *scene, uint32_t frame_begin, uint32_t frame_count, int f
  * a launch.  VS_SCHEDULE_PERSISTENT: one resident wave of warps that keep 32
  * paths in flight each and refill the lanes of finished paths after every
  * bounce (path regeneration).  VS_SCHEDULE_WAVEFRONT: waves of up to
- * 16,777,216 paths whose bounces run as separate kernels (traversal, shading
- * sorted by material) over path state in device memory (208 bytes per path
- * slot, allocated on first use; smaller waves where memory is short). */
+ * 16,777,216 paths (4,194,304 where device memory is not plentiful) whose
+ * bounces run as separate kernels (traversal, shading sorted by material) over
+ * path state in device memory (216 bytes per path slot, allocated on first
+ * use). */
 #define VS_SCHEDULE_GRID 0
 #define VS_SCHEDULE_PERSISTENT 1
 #define VS_SCHEDULE_WAVEFRONT 2

@@ -405,7 +405,8 @@ def test_schedules_give_the_same_film(vb, gpu_ctx, case):
     elif case == 'dimension1':
         sc = scenes.box_room(width=33, height=31, dimension=1)
     else:
-        # 5 frames of 1024 x 1024 exceed one wavefront wave (2^22 paths).
+        # 5 frames of 1024 x 1024 exceed one wave of 2^22 path slots (the
+        # binned schedule's; the unbinned one's where memory is short).
         sc = scenes.box_room(width=1024, height=1024, max_depth=4, sampler='pcg')
     films = {}
     for schedule in ('grid', 'persistent', 'wavefront', 'wavefront_binned'):

@@ -108,10 +108,12 @@ def test_one_wavelength(vb, gpu_ctx, room):
 
 
 def test_film_across_waves(vb, gpu_ctx):
-    # 17 x 2^20 paths: one full wave of 2^24 path slots and a second, smaller one.
-    sc = scenes.box_room(width=1024, height=1024, max_depth=2)
-    (grid, _), (film, _) = _films(vb, gpu_ctx, sc, 17, ['grid', 'wavefront'])
+    # 17 x 2^20 paths: one full wave of 2^24 path slots and a second, smaller
+    # one; five waves of the binned schedule.
+    sc = scenes.box_room(width=1024, height=1024, max_depth=5)
+    (grid, _), (film, _), (binned, _) = _films(vb, gpu_ctx, sc, 17, ['grid', 'wavefront', 'wavefront_binned'])
     assert np.array_equal(grid, film)
+    assert np.array_equal(grid, binned)
 
 
 def _lens(sc):

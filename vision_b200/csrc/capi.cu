@@ -1,8 +1,10 @@
 // extern "C" boundary of libvision_b200.so (declared in include/vision_b200.h).
 #include "../../include/vision_b200.h"
 
+#include <atomic>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <stdexcept>
 #include <string>
@@ -25,6 +27,9 @@ struct vs_context {
     mutable std::mutex mu;
     std::string error;
     bool consts_uploaded = false;
+    // Device memory of the scenes' wide path slots (shared: a scene may be
+    // destroyed after its context).
+    std::shared_ptr<std::atomic<uint64_t>> wide_bytes = std::make_shared<std::atomic<uint64_t>>(0);
     HostCopy download;  // films and frame buffers to host memory
 };
 
@@ -91,7 +96,7 @@ struct vs_scene {
     int schedule = VS_SCHEDULE_AUTO;
     // Whether real-time and cached frames run as wavefront passes.
     bool wavefront_frames() const { return schedule == VS_SCHEDULE_AUTO || schedule == VS_SCHEDULE_WAVEFRONT; }
-    // Path slots of the wavefront schedule.
+    // Path slots of the wavefront passes.
     struct WfBufs {
         DevBuf<float4> o, d, tp, lam, pdf, L, sh_o, sh_d, sh_c;
         DevBuf<uint4> st;
@@ -158,7 +163,13 @@ struct vs_scene {
             }
             return b;
         }
-    } wf;
+    };
+    // Slots of real-time and cached frames and of vs_render's waves of up to
+    // kWfSlots, and of its larger ones (render_slots).
+    WfBufs wf, wide;
+    bool wide_refused = false;
+    std::shared_ptr<std::atomic<uint64_t>> wide_total;  // the context's
+    uint64_t wide_bytes() const { return static_cast<uint64_t>(wide.capacity) * kWfBytesPerSlot; }
     // Cache-terminated rendering: per-pixel queries, training samples, the
     // material albedo/roughness table of the feature encoding.
     struct CacheBufs {
@@ -291,6 +302,8 @@ struct vs_scene {
         tex_texels.free(); textures.free();
         filter_tab.free(); filter_alias.free(); tlas_inst.free(); inst_xf.free();
         film32.free(); exposed.free(); film64.free(); radiance.free(); path_counter.free(); wf.free();
+        if (wide_total) *wide_total -= wide_bytes();
+        wide.free();
         rt.free();
         svgf.free();
         cachebuf.free();
@@ -378,16 +391,15 @@ namespace {
 // Upper bound on paths per megakernel launch; sizes the radiance scratch
 // (16 bytes per path).
 constexpr uint64_t kMaxPathsPerLaunch = 1ull << 26;
-// Path slots of one wavefront wave of vs_render (208 B each: 3.25 GiB).  Every
-// wave ends in bounces of few paths that last as long as their slowest warps
-// (about 2 ms over the 16 bounces of the large scene), so waves are large:
-// 8.4 M paths of that scene took 26.2 ms in two waves and 22.5 ms in one.
-constexpr uint64_t kWfWaveSlots = 1ull << 24;
-// Where device memory is short the waves shrink, to this at the least.
-constexpr uint64_t kWfMinWaveSlots = 1ull << 22;
-// Pixels up to which real-time and cached frames run in wavefront form (one
-// path slot per pixel).
-constexpr uint64_t kWfFramePixels = 1ull << 22;
+// Path slots of a wavefront wave (216 B each: 0.84 GiB), and the pixels up to
+// which real-time and cached frames run in wavefront form (a slot per pixel).
+constexpr uint64_t kWfSlots = 1ull << 22;
+// Slots of vs_render's wide waves (3.4 GiB), where device memory is plentiful.
+// Every wave ends in bounces of few paths that last as long as their slowest
+// warps (about 2 ms over the 16 bounces of the large scene), so fewer and
+// larger waves are faster: 8.4 M paths of that scene took 26.2 ms in two waves
+// and 22.5 ms in one.
+constexpr uint64_t kWfWideSlots = 1ull << 24;
 
 int fail(const vs_context *ctx, int code, const std::string &msg) {
     if (ctx) {
@@ -463,6 +475,43 @@ bool small_render(const HostScene &h, uint64_t paths) {
     if (!diffuse && h.ip.srgb) return false;
     if (h.ip.spectrum_dim < 2u && (!diffuse || h.has_env)) return false;
     return paths <= std::min<uint64_t>(h.ip.max_depth, 16u) * (diffuse ? 7168u : 1536u);
+}
+
+// The path slots of vs_render's waves for `paths` paths (on success *out names
+// them).  More paths than kWfSlots get wide waves, of 2^23 or 2^24 slots so
+// that growing renders allocate at most twice, while memory is plentiful: half
+// of the device stays free and the wide slots of a context's scenes together
+// take at most a sixteenth of it.  So a device that is short, or shared with
+// other programs or with many scenes, spends what kWfSlots waves need.  A scene
+// that was refused keeps its smaller waves: nothing is freed and tried again on
+// later calls, which would synchronise the device each time.
+cudaError_t render_slots(vs_scene *s, uint64_t paths, bool binned, vs_scene::WfBufs **out) {
+    *out = &s->wf;
+    if (paths > kWfSlots && !binned) {
+        const uint64_t n = paths > kWfWideSlots / 2 ? kWfWideSlots : kWfWideSlots / 2;
+        if (s->wide.capacity < n && !s->wide_refused) {
+            const uint64_t held = s->wide_bytes(), more = n * kWfBytesPerSlot - held;
+            size_t free_bytes = 0, total = 0;
+            cudaError_t e = cudaMemGetInfo(&free_bytes, &total);
+            if (e != cudaSuccess) return e;
+            if (!s->wide_total) s->wide_total = s->ctx->wide_bytes;
+            const bool room = free_bytes >= more + total / 2;
+            if (room && s->wide_total->fetch_add(more) + more <= total / 16) {
+                if (s->wide.ensure(static_cast<uint32_t>(n), false) != cudaSuccess) {
+                    (void)cudaGetLastError();
+                    *s->wide_total -= held + more;
+                }
+            } else if (room) {
+                *s->wide_total -= more;
+            }
+            s->wide_refused = s->wide.capacity < n;
+        }
+        if (s->wide.capacity != 0) {
+            *out = &s->wide;
+            return cudaSuccess;
+        }
+    }
+    return s->wf.ensure(static_cast<uint32_t>(std::min(paths, kWfSlots)), binned);
 }
 
 // Per instance: the world-to-object rows and (mesh root node, first
@@ -867,17 +916,8 @@ int vs_render(vs_scene *s, uint32_t frame_begin, uint32_t frame_count, int film_
     const bool wavefront = schedule == VS_SCHEDULE_WAVEFRONT || binned;
     if (!wavefront && has_mix(s->host))
         return fail(ctx, VS_E_UNSUPPORTED, "mix / add materials render with the wavefront schedules only");
-    if (wavefront) {
-        uint64_t slots = std::min<uint64_t>(frames_per_chunk * npix, kWfWaveSlots);
-        cudaError_t e;
-        while ((e = s->wf.ensure(static_cast<uint32_t>(slots), binned)) ==
-                   cudaErrorMemoryAllocation &&
-               slots > kWfMinWaveSlots) {
-            (void)cudaGetLastError();
-            slots = std::max(slots / 2, kWfMinWaveSlots);
-        }
-        VS_CUDA(e, "wavefront slots alloc");
-    }
+    vs_scene::WfBufs *slots = nullptr;
+    if (wavefront) VS_CUDA(render_slots(s, frames_per_chunk * npix, binned, &slots), "wavefront slots alloc");
     DeviceScene dv = s->device_view();
     auto timed_event = [&](std::vector<cudaEvent_t> &v) -> cudaError_t {
         cudaEvent_t e;
@@ -892,7 +932,7 @@ int vs_render(vs_scene *s, uint32_t frame_begin, uint32_t frame_count, int film_
         if (wavefront) {
             unsigned n = 0;
             VS_CUDA(launch_render_wavefront(dv, frame_begin + f, fc, s->radiance.ptr,
-                                            binned ? s->wf.view_binned() : s->wf.view(),
+                                            binned ? slots->view_binned() : slots->view(),
                                             shading_classes(s->host), st, &n),
                     "wavefront render");
             add_launches(n);
@@ -1307,7 +1347,7 @@ int restir_frame_locked(vs_scene *s, uint32_t frame_index, uint32_t film_index, 
     if (s->timing) VS_CUDA(timed_event(s->ev_render), "timing event");
     unsigned n = 0;
     const uint64_t rt_npix = static_cast<uint64_t>(p.width) * p.height;
-    const bool wavefront = s->wavefront_frames() && rt_npix <= kWfFramePixels;
+    const bool wavefront = s->wavefront_frames() && rt_npix <= kWfSlots;
     WfBuffers wfv{};
     if (wavefront) {
         VS_CUDA(s->wf.ensure(static_cast<uint32_t>(rt_npix), false), "wavefront slots alloc");
@@ -1368,7 +1408,7 @@ int restir_prepare_locked(vs_scene *s) {
     rc = rt_ensure(s, ctx->stream);
     if (rc != VS_OK) return rc;
     const uint64_t npix = static_cast<uint64_t>(s->host.cam.width) * s->host.cam.height;
-    if (s->wavefront_frames() && npix <= kWfFramePixels) {
+    if (s->wavefront_frames() && npix <= kWfSlots) {
         VS_CUDA(s->wf.ensure(static_cast<uint32_t>(npix), false), "wavefront slots alloc");
         VS_CUDA(s->radiance.alloc(npix), "radiance alloc");
     }
@@ -1858,7 +1898,7 @@ int vs_render_cached(vs_scene *s, vs_cache *c, uint32_t frame_begin, uint32_t fr
     p.query_depth = 2;
     p.suffix_depth = 2;
     // Wavefront frames need one path slot per pixel.
-    const bool wavefront = s->wavefront_frames() && npix <= kWfFramePixels;
+    const bool wavefront = s->wavefront_frames() && npix <= kWfSlots;
     if (wavefront) {
         VS_CUDA(s->wf.ensure(npix, false), "wavefront slots alloc");
         VS_CUDA(s->radiance.alloc(npix), "radiance alloc");
