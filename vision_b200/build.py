@@ -40,7 +40,7 @@ def nvcc():
 def _digest(paths, extra):
     h = hashlib.sha256()
     for p in paths:
-        h.update(p.encode())
+        h.update(os.path.relpath(p, HERE).encode())  # the same in a copy of the tree elsewhere
         with open(p, 'rb') as f:
             h.update(f.read())
     h.update(' '.join(extra).encode())
