@@ -27,6 +27,7 @@
 // albedo (3); sin/cos(2^k pi u) of the hero wavelength u = (lambda_0 - 360) /
 // 470 for k = 0..2 (6).
 #include "vs_cache_render.h"
+#include "vs_resident.h"
 #include "vs_wavefront.cuh"
 #include "vs_launch.h"
 
@@ -477,22 +478,11 @@ __global__ void __launch_bounds__(128) k_cache_suffix(const __grid_constant__ De
 
 namespace {
 
-template <typename K>
-unsigned wave_grid(K kernel) {
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0);
-    return static_cast<unsigned>(std::max(1, sms * std::max(per_sm, 1)));
-}
-
 template <uint32_t C>
 void cw_shade(uint32_t mask, const DeviceScene &s, const WfBuffers &b, uint32_t cur, float4 *ended, cudaStream_t st,
               unsigned &n) {
-    static unsigned grid = 0;
     if (!((mask >> C) & 1u)) return;
-    if (!grid) grid = wave_grid(k_cw_shade<C>);
-    k_cw_shade<C><<<grid, 128, 0, st>>>(s, b, cur, ended);
+    k_cw_shade<C><<<wave_grid<k_cw_shade<C>>(), 128, 0, st>>>(s, b, cur, ended);
     ++n;
 }
 
@@ -504,22 +494,16 @@ cudaError_t launch_cache_frame_wavefront(const DeviceScene &s, const CacheFrameP
                                          uint32_t *suffix_count, cudaStream_t st, unsigned *launches) {
     const uint32_t npix = s.cam.width * s.cam.height;
     if (npix > b.capacity) return cudaErrorInvalidValue;
-    static unsigned g_gen = 0, g_trace = 0, g_trace2 = 0, g_query = 0, g_suffix = 0;
-    if (!g_gen) {
-        g_gen = wave_grid(k_cw_generate);
-        g_trace = wave_grid(k_cw_trace<kLevelsFlat>);
-        g_trace2 = wave_grid(k_cw_trace<kLevelsTwo>);
-        g_query = wave_grid(k_cache_query);
-        g_suffix = wave_grid(k_cache_suffix);
-    }
+    const unsigned g_gen = wave_grid<k_cw_generate>(), g_query = wave_grid<k_cache_query>();
+    const unsigned g_suffix = wave_grid<k_cache_suffix>();
     // The prefix ends at the query vertex, not at the scene's depth limit
     // (k_cache_paths does not apply it either).
     DeviceScene sv = s;
     sv.ip.max_depth = 0xffffffffu;
     const bool two = s.two_level != 0u;
     auto trace = [&](uint32_t round) {
-        if (two) k_cw_trace<kLevelsTwo><<<g_trace2, 128, 0, st>>>(sv, b, round, ended);
-        else k_cw_trace<kLevelsFlat><<<g_trace, 128, 0, st>>>(sv, b, round, ended);
+        if (two) k_cw_trace<kLevelsTwo><<<wave_grid<k_cw_trace<kLevelsTwo>>(), 128, 0, st>>>(sv, b, round, ended);
+        else k_cw_trace<kLevelsFlat><<<wave_grid<k_cw_trace<kLevelsFlat>>(), 128, 0, st>>>(sv, b, round, ended);
     };
     cudaError_t e = cudaMemsetAsync(p.q_rec, 0, sizeof(CacheQueryRec) * npix, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(suffix_count, 0, sizeof(uint32_t), st);

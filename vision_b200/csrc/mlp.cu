@@ -32,6 +32,7 @@
 // records the error, skips the rest of its work, frees its tensor memory and
 // returns.
 #include "vs_mlp.h"
+#include "vs_resident.h"
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -659,8 +660,6 @@ __global__ void k_mlp_adam(float *w, float *m, float *v, const float *g, MlpAdam
     pack[pack_offset(l, in, out)] = u;
 }
 
-int g_sm_count = 0;
-
 }  // namespace
 
 cudaError_t mlp_pack(const MlpState &s, cudaStream_t st) {
@@ -668,43 +667,34 @@ cudaError_t mlp_pack(const MlpState &s, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-static cudaError_t sm_count(int &n) {
-    if (g_sm_count == 0) {
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess) return e;
-    }
-    n = g_sm_count;
-    return cudaSuccess;
-}
-
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
 // against the driver library).
-static PFN_cuTensorMapEncodeTiled_v12000 g_encode_tiled = nullptr;
-
-static cudaError_t encode_fn() {
-    if (g_encode_tiled) return cudaSuccess;
+static cudaError_t encode_fn(PFN_cuTensorMapEncodeTiled_v12000 *out) {
+    static std::atomic<PFN_cuTensorMapEncodeTiled_v12000> found{nullptr};
+    *out = found.load();
+    if (*out) return cudaSuccess;
     void *fn = nullptr;
     cudaDriverEntryPointQueryResult q;
     cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q);
     if (e != cudaSuccess) return e;
     if (q != cudaDriverEntryPointSuccess || !fn) return cudaErrorSymbolNotFound;
-    g_encode_tiled = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+    *out = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+    found.store(*out);
     return cudaSuccess;
 }
 
 // The feature matrix (n rows of 64 BF16, 128-byte rows, 16-byte aligned) as a
 // TMA tensor map with 128-row x 64-column boxes and the 128-byte swizzle.
 static cudaError_t feature_map(const uint16_t *feat, uint32_t n, CUtensorMap *map) {
-    cudaError_t e = encode_fn();
+    PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
+    cudaError_t e = encode_fn(&encode);
     if (e != cudaSuccess) return e;
     if (reinterpret_cast<uintptr_t>(feat) & 15u) return cudaErrorMisalignedAddress;
     cuuint64_t dims[2] = {64u, n};
     cuuint64_t strides[1] = {128u};
     cuuint32_t box[2] = {64u, static_cast<cuuint32_t>(kTile)};
     cuuint32_t elem[2] = {1u, 1u};
-    CUresult r = g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t *>(feat), dims, strides,
+    CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t *>(feat), dims, strides,
                                 box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
@@ -712,17 +702,13 @@ static cudaError_t feature_map(const uint16_t *feat, uint32_t n, CUtensorMap *ma
 
 cudaError_t mlp_infer(const MlpState &s, const uint16_t *feat, uint32_t n, float4 *out, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    static bool attr = false;
-    if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(k_mlp_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, kInferSmem);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    cudaError_t e = allow_shared<k_mlp_infer>(kInferSmem);
+    if (e != cudaSuccess) return e;
     CUtensorMap map;
-    cudaError_t e = feature_map(feat, n, &map);
+    e = feature_map(feat, n, &map);
     if (e != cudaSuccess) return e;
     int sms = 0;
-    e = sm_count(sms);
+    e = device_sms(&sms);
     if (e != cudaSuccess) return e;
     const uint32_t tiles = (n + kTile - 1) / kTile;
     uint32_t grid = static_cast<uint32_t>(sms);
@@ -734,18 +720,14 @@ cudaError_t mlp_infer(const MlpState &s, const uint16_t *feat, uint32_t n, float
 
 cudaError_t mlp_train_step(const MlpState &s, const uint16_t *feat, const float4 *target, uint32_t n, MlpAdam adam,
                            bool update, cudaStream_t st) {
-    static bool attr = false;
-    if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem);
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    cudaError_t e = allow_shared<k_mlp_train>(kTrainSmem);
+    if (e != cudaSuccess) return e;
     // The loss follows the gradient: one clear for both.
-    cudaError_t e = cudaMemsetAsync(s.grad, 0, kMlpGradBytes, st);
+    e = cudaMemsetAsync(s.grad, 0, kMlpGradBytes, st);
     if (e != cudaSuccess) return e;
     if (n > 0) {
         int sms = 0;
-        e = sm_count(sms);
+        e = device_sms(&sms);
         if (e != cudaSuccess) return e;
         uint32_t tiles = (n + kTile - 1) / kTile;
         uint32_t grid = static_cast<uint32_t>(sms);

@@ -22,6 +22,7 @@
 // wavelengths: the reference's ReSTIR code moves spectra through float3
 // (SampledSpectrum::vec3, SampledSpectrum(Float3)), which is only defined for
 // three channels.
+#include "vs_resident.h"
 #include "vs_wavefront.cuh"
 #include "vs_launch.h"
 #include "vs_restir.h"
@@ -1718,19 +1719,6 @@ cudaError_t launch_rt_reset(uint32_t npix, const RtBuffers &b, cudaStream_t st) 
     return cudaGetLastError();
 }
 
-namespace {
-
-template <typename K>
-unsigned rt_wave_grid(K kernel) {
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0);
-    return static_cast<unsigned>(std::max(1, sms * std::max(per_sm, 1)));
-}
-
-}  // namespace
-
 cudaError_t launch_rt_frame(const DeviceScene &s, const RtParams &p, const RtBuffers &b, uint32_t film_index,
                             float4 *film, const WfBuffers *wf, float4 *radiance, uint32_t class_mask, cudaStream_t st,
                             unsigned *launches) {
@@ -1739,20 +1727,13 @@ cudaError_t launch_rt_frame(const DeviceScene &s, const RtParams &p, const RtBuf
     unsigned n = 0;
     if (p.M_bsdf <= 1u && b.di_stage) {
         // One resident wave of each list kernel (its own occupancy).
-        static unsigned g_lights = 0, g_trace = 0, g_eval = 0, g_vis = 0;
-        if (!g_lights) {
-            g_lights = rt_wave_grid(k_di_lights);
-            g_trace = rt_wave_grid(k_di_bsdf_trace);
-            g_eval = rt_wave_grid(k_di_bsdf_eval);
-            g_vis = rt_wave_grid(k_di_visibility);
-        }
         cudaError_t e = cudaMemsetAsync(b.di_count, 0, 3 * sizeof(uint32_t), st);
         if (e != cudaSuccess) return e;
         k_di_primary<<<grid, block, 0, st>>>(s, p, b);
-        k_di_lights<<<g_lights, 128, 0, st>>>(s, p, b);
-        k_di_bsdf_trace<<<g_trace, 128, 0, st>>>(s, p, b);
-        k_di_bsdf_eval<<<g_eval, 128, 0, st>>>(s, p, b);
-        k_di_visibility<<<g_vis, 128, 0, st>>>(s, b);
+        k_di_lights<<<wave_grid<k_di_lights>(), 128, 0, st>>>(s, p, b);
+        k_di_bsdf_trace<<<wave_grid<k_di_bsdf_trace>(), 128, 0, st>>>(s, p, b);
+        k_di_bsdf_eval<<<wave_grid<k_di_bsdf_eval>(), 128, 0, st>>>(s, p, b);
+        k_di_visibility<<<wave_grid<k_di_visibility>(), 128, 0, st>>>(s, b);
         k_di_temporal<<<grid, block, 0, st>>>(s, p, b);
         n += 6;
     } else {
@@ -1760,29 +1741,15 @@ cudaError_t launch_rt_frame(const DeviceScene &s, const RtParams &p, const RtBuf
         ++n;
     }
     if (p.di.open) {
-        static unsigned g_vis = 0, g_shade = 0;
-        if (!g_vis) {
-            g_vis = rt_wave_grid(k_di_sp_vis);
-            g_shade = rt_wave_grid(k_di_sp_shade);
-        }
         cudaError_t e = cudaMemsetAsync(b.di_count, 0, 3 * sizeof(uint32_t), st);
         if (e != cudaSuccess) return e;
         k_di_sp_combine<<<grid, block, 0, st>>>(s, p, b);
-        k_di_sp_vis<<<g_vis, 128, 0, st>>>(s, b);
-        k_di_sp_shade<<<g_shade, 128, 0, st>>>(s, p, b);
+        k_di_sp_vis<<<wave_grid<k_di_sp_vis>(), 128, 0, st>>>(s, b);
+        k_di_sp_shade<<<wave_grid<k_di_sp_shade>(), 128, 0, st>>>(s, p, b);
         n += 3;
     }
     if (wf && radiance) {
-        static unsigned g_ext = 0, g_shade[kWfClasses] = {};
-        if (!g_ext) {
-            g_ext = rt_wave_grid(k_gi_wf_trace);
-            g_shade[0] = rt_wave_grid(k_gi_wf_shade<0>);
-            g_shade[1] = rt_wave_grid(k_gi_wf_shade<1>);
-            g_shade[3] = rt_wave_grid(k_gi_wf_shade<3>);
-            g_shade[4] = rt_wave_grid(k_gi_wf_shade<4>);
-            g_shade[5] = rt_wave_grid(k_gi_wf_shade<5>);
-            g_shade[6] = rt_wave_grid(k_gi_wf_shade<6>);
-        }
+        const unsigned g_ext = wave_grid<k_gi_wf_trace>();
         const uint32_t np = p.width * p.height;
         const unsigned g_pix = (np + 127) / 128;
         const uint32_t mask = class_mask | 1u;
@@ -1799,12 +1766,12 @@ cudaError_t launch_rt_frame(const DeviceScene &s, const RtParams &p, const RtBuf
                 k_gi_wf_first<<<g_ext, 128, 0, st>>>(s, b, *wf);
                 ++n;
             }
-            if (mask & 1u) { k_gi_wf_shade<0><<<g_shade[0], 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
-            if (mask & 2u) { k_gi_wf_shade<1><<<g_shade[1], 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
-            if (mask & 8u) { k_gi_wf_shade<3><<<g_shade[3], 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
-            if (mask & 16u) { k_gi_wf_shade<4><<<g_shade[4], 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
-            if (mask & 32u) { k_gi_wf_shade<5><<<g_shade[5], 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
-            if (mask & 64u) { k_gi_wf_shade<6><<<g_shade[6], 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
+            if (mask & 1u) { k_gi_wf_shade<0><<<wave_grid<k_gi_wf_shade<0>>(), 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
+            if (mask & 2u) { k_gi_wf_shade<1><<<wave_grid<k_gi_wf_shade<1>>(), 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
+            if (mask & 8u) { k_gi_wf_shade<3><<<wave_grid<k_gi_wf_shade<3>>(), 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
+            if (mask & 16u) { k_gi_wf_shade<4><<<wave_grid<k_gi_wf_shade<4>>(), 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
+            if (mask & 32u) { k_gi_wf_shade<5><<<wave_grid<k_gi_wf_shade<5>>(), 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
+            if (mask & 64u) { k_gi_wf_shade<6><<<wave_grid<k_gi_wf_shade<6>>(), 128, 0, st>>>(s, *wf, cur, radiance); ++n; }
         }
         k_gi_wf_finish<<<g_pix, 128, 0, st>>>(s, p, b, radiance);
         ++n;
@@ -1814,12 +1781,10 @@ cudaError_t launch_rt_frame(const DeviceScene &s, const RtParams &p, const RtBuf
     }
     k_gi_temporal<<<grid, block, 0, st>>>(s, p, b);
     {
-        static unsigned g_vis = 0;
-        if (!g_vis) g_vis = rt_wave_grid(k_gi_sp_vis);
         cudaError_t e = cudaMemsetAsync(b.gs_count, 0, 2 * sizeof(uint32_t), st);
         if (e != cudaSuccess) return e;
         k_gi_sp_select<<<grid, block, 0, st>>>(s, p, b);
-        k_gi_sp_vis<<<g_vis, 128, 0, st>>>(s, b);
+        k_gi_sp_vis<<<wave_grid<k_gi_sp_vis>(), 128, 0, st>>>(s, b);
         k_gi_sp_combine<<<grid, block, 0, st>>>(s, p, b);
         n += 2;
     }
