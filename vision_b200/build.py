@@ -43,7 +43,7 @@ def _digest(paths, extra):
         h.update(os.path.relpath(p, HERE).encode())  # the same in a copy of the tree elsewhere
         with open(p, 'rb') as f:
             h.update(f.read())
-    h.update(' '.join(extra).encode())
+    h.update(' '.join(os.path.relpath(x, HERE) if os.path.isabs(x) else x for x in extra).encode())
     return h.hexdigest()
 
 
