@@ -13,7 +13,7 @@ from vision_b200 import scenes
 
 pytestmark = pytest.mark.gpu
 
-SMALLEST = (3 << 20) // 16  # pixels of a linear film: the smallest threaded copy
+PIXELS_1MB = (1 << 20) // 16  # of a linear film: the smallest threaded copy
 CHUNK = (512 << 10) // 16
 RING = 8 * CHUNK
 
@@ -28,7 +28,7 @@ def _download(vb, s, address, pixels, which=0):
     s.ctx.check(vb.lib.vs_film_download(s.handle, ctypes.c_void_p(address), pixels * 16, which), 'film_download')
 
 
-@pytest.mark.parametrize('pixels', [SMALLEST - 1, SMALLEST, SMALLEST + 1, RING - CHUNK - 1, RING - CHUNK + 1, RING - 1, RING,
+@pytest.mark.parametrize('pixels', [PIXELS_1MB - 1, PIXELS_1MB, PIXELS_1MB + 1, 3 * CHUNK - 1, 3 * CHUNK + 1, RING - 1, RING,
                                     RING + 1, RING + CHUNK, RING + CHUNK + 1, 3 * RING + 5])
 def test_threaded_copy_equals_direct_copy(vb, gpu_ctx, pixels):
     width = pixels if pixels < 1 << 16 else next(w for w in range(1 << 15, 0, -1) if pixels % w == 0)

@@ -14,12 +14,11 @@ namespace vs {
 namespace {
 constexpr size_t kSlots = 8;
 constexpr size_t kChunk = 512u << 10;
-// Below this the threads' wake-up costs what they save or more.  Film downloads
-// after a render, medians on 16 cores, one thread / several: 1.05 MB 0.22 to
-// 0.30 / 0.27 ms, 1.4 MB 0.34 / 0.32 to 0.36, 2.1 MB 0.35 to 0.48 / 0.41 to 0.45,
-// 2.8 MB 0.43 to 0.50 / 0.46, 3.2 MB 0.47 to 0.55 / 0.45 to 0.48, 3.6 MB 0.54 to
-// 0.57 / 0.41, 4.2 MB 0.65 / 0.35, 17 MB 2.2 / 1.1, 33 MB 4.2 / 2.6.
-constexpr size_t kMinBytes = 3u << 20;
+// Below this the threads' wake-up costs what they save.  Film downloads after a
+// render, measured on 16 cores, one thread / several: 1.05 MB 0.24 / 0.13 to
+// 0.27 ms, 3.2 MB 0.57 / 0.35 to 0.47, 4.9 MB 0.82 / 0.38, 17 MB 2.17 / 1.09,
+// 33 MB 4.08 / 2.47.
+constexpr size_t kMinBytes = 1u << 20;
 constexpr unsigned kMaxHelpers = 3;
 }  // namespace
 
