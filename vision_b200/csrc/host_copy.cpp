@@ -14,10 +14,13 @@ namespace vs {
 namespace {
 constexpr size_t kSlots = 8;
 constexpr size_t kChunk = 512u << 10;
-// Below this the threads' wake-up costs what they save.  Film downloads after a
-// render, measured on 16 cores, one thread / several: 1.05 MB 0.24 / 0.13 to
-// 0.27 ms, 3.2 MB 0.57 / 0.35 to 0.47, 4.9 MB 0.82 / 0.38, 17 MB 2.17 / 1.09,
-// 33 MB 4.08 / 2.47.
+// Below this the threads' wake-up costs what they save.  Into arrays whose pages
+// are new, as a program's that keeps its films, on 16 cores, one thread / several:
+// a box room and its 1.05 MB film 1.92 / 1.84 ms, a principled room and its films
+// of 1.4 and 2.8 MB 2.14 / 1.89.  Into memory that the last film's array has just
+// given back: 1.05 MB 0.22 to 0.30 / 0.27 ms, 2.1 MB 0.35 to 0.48 / 0.41 to 0.45,
+// 2.8 MB 0.43 to 0.50 / 0.46, 3.6 MB 0.54 to 0.57 / 0.41, 4.2 MB 0.65 / 0.35, 17 MB
+// 2.2 / 1.1, 33 MB 4.2 / 2.6.
 constexpr size_t kMinBytes = 1u << 20;
 constexpr unsigned kMaxHelpers = 3;
 }  // namespace
