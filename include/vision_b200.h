@@ -88,6 +88,8 @@ int vs_version(void);
 /* Creates a context on CUDA device `device`; device = -1 makes a host-only
  * context that can parse, build and export scenes but not render. */
 int vs_context_create(int device, vs_context **out);
+/* Scenes and caches of the context may be destroyed after it, and are good for
+ * nothing else then. */
 void vs_context_destroy(vs_context *ctx);
 /* Message of the last failed call on this context (never NULL). */
 const char *vs_last_error(const vs_context *ctx);

@@ -66,6 +66,7 @@ struct DevBuf {
 
 struct vs_scene {
     vs_context *ctx = nullptr;
+    int device = -1;  // the context's, for the destructor (which may run after the context's)
     std::mutex mu;
     HostScene host;
     bool built = false;
@@ -684,6 +685,7 @@ int vs_scene_load_json(vs_context *ctx, const char *json, size_t len, const char
     *out = nullptr;
     vs_scene *s = new vs_scene();
     s->ctx = ctx;
+    s->device = ctx->device;
     try {
         load_scene_json(std::string(json, len), base_dir ? base_dir : "", table_cache ? table_cache : "", s->host);
     } catch (const std::exception &e) {
@@ -698,7 +700,7 @@ int vs_scene_load_json(vs_context *ctx, const char *json, size_t len, const char
 
 void vs_scene_destroy(vs_scene *s) {
     if (!s) return;
-    if (s->ctx && s->ctx->device >= 0) cudaSetDevice(s->ctx->device);
+    if (s->device >= 0) cudaSetDevice(s->device);
     delete s;
 }
 
@@ -1683,10 +1685,11 @@ const char *vs_server_last_error(const vs_server *s) {
 
 struct vs_cache {
     vs_context *ctx = nullptr;
+    int device = -1;  // as vs_scene's
     MlpState st{};
     MlpAdam adam{1e-3f, 0.9f, 0.999f, 1e-8f, 1u, 0.0f};
     ~vs_cache() {
-        if (ctx && ctx->device >= 0) cudaSetDevice(ctx->device);
+        if (device >= 0) cudaSetDevice(device);
         cudaFree(st.w);
         cudaFree(st.pack);
         cudaFree(st.m);
@@ -1715,6 +1718,7 @@ int vs_cache_create(vs_context *ctx, uint64_t seed, vs_cache **out) {
     VS_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
     vs_cache *c = new vs_cache();
     c->ctx = ctx;
+    c->device = ctx->device;
     MlpState &s = c->st;
     cudaError_t e = cudaMalloc(&s.w, sizeof(float) * kMlpParams);
     if (e == cudaSuccess) e = cudaMalloc(&s.pack, sizeof(uint16_t) * kMlpPackElems);
