@@ -74,18 +74,17 @@ DEFAULT_STEPS = {'box_room': 100, 'large_scene': 5, 'many_lights': 64, 'serving'
 # dram__bytes_write.sum of one launch divided by its paths; profiles/).
 NCU_TRAFFIC_PER_PATH = {('large_scene', 'persistent'): 383.6e6 / 2097152,
                         ('box_room', 'persistent'): 7.42e6 / 1048576,
-                        # all wavefront kernels of one render (2,097,152 and 1,048,576 paths)
-                        ('large_scene', 'wavefront'): 3059.95e6 / 2097152,
-                        ('box_room', 'wavefront'): 1990.0e6 / 1048576}
+                        # all wavefront kernels of one render of the workload
+                        ('large_scene', 'wavefront'): 101955.5e6 / 67108864,
+                        ('box_room', 'wavefront'): 2258.8e6 / 1048576}
 
 # Issue-slot utilisation and active threads per instruction of the dominant
 # traversal kernel, from the committed one-kernel ncu capture of the same
 # workload's 2-spp case (the binding measure of the L1/L2-resident traversal).
 NCU_ISSUE = {('large_scene', 'wavefront'): {
-    'issue_active': 0.652, 'threads_per_inst': 12.95,
-    'issue_source': 'ncu sm__inst_issued / smsp__thread_inst_executed_per_inst_executed of k_wf_extend, '
-                    'the closest-hit pass before path and shadow rays shared k_wf_trace '
-                    '(profiles/k_wf_extend_large_scene.md)'}}
+    'issue_active': 0.679, 'threads_per_inst': 12.77,
+    'issue_source': 'ncu smsp__issue_active / smsp__thread_inst_executed_per_inst_executed of k_wf_trace '
+                    '(profiles/k_wf_trace_large_scene.md)'}}
 
 # Algorithmic bytes per pixel-frame of the ReSTIR frame, from the record sizes
 # (64 B surfaces and reservoirs, 32 B extensions and BSDF samples, 16 B
@@ -457,6 +456,7 @@ def run_plain(args, w, rank, world, local_rank, dist):
     peak, peak_src = measured_peaks()
     kernel_s = render_ms / 1e3 / max(render_launches, 1)
     achieved = bytes_per_path * paths_per_step / kernel_s / 1e9
+    dram_per_path = NCU_TRAFFIC_PER_PATH.get((args.workload, args.schedule))
     line = {
         'metric': 'Mpaths/s', 'value': value, 'unit': 'Mpaths/s', 'n_gpus': world, 'steps': args.steps,
         'warmup': args.warmup, 'ms_per_step': step_ms / args.steps, 'higher_is_better': True, 'scaling': 'weak',
@@ -468,11 +468,13 @@ def run_plain(args, w, rank, world, local_rank, dist):
                    'schedule': args.schedule},
         'roofline': {'bound': 'hbm', 'achieved': achieved, 'peak': peak, 'unit': 'GB/s', 'frac': achieved / peak,
                      'peak_source': peak_src,
-                     'traffic': (NCU_TRAFFIC_PER_PATH[(args.workload, args.schedule)] * paths_per_step * args.steps /
-                                 max(render_launches, 1)
-                                 if (args.workload, args.schedule) in NCU_TRAFFIC_PER_PATH else None),
+                     'achieved_source': 'node, triangle and hit records fetched (counted by an instrumented render) '
+                                        'per kernel time; most come from L1 and L2',
+                     'traffic': (dram_per_path * paths_per_step * args.steps / max(render_launches, 1)
+                                 if dram_per_path else None),
                      'traffic_source': 'ncu dram bytes per path of the committed profile (all kernels of the '
                                        'schedule for one render) x paths per launch',
+                     'dram_gbs': (dram_per_path * paths_per_step / kernel_s / 1e9 if dram_per_path else None),
                      'kernel': {'persistent': 'k_render_regen', 'grid': 'k_render',
                                 'wavefront': 'wavefront (k_wf_trace, k_wf_shade)',
                                 'wavefront_binned': 'wavefront (k_wf_trace, k_wf_shade; binned rays)'}[
